@@ -179,7 +179,8 @@ int launch_stage(nb_instance* h, const float* const in[4], const float* const u0
     L.nstars_host = h->nstars;
     L.order = h->tile_order;
     L.no_sources = no_sources ? 1 : 0;
-    L.idx32 = h->ncell < (1LL << 31) ? 1 : 0;
+    L.idx32 = nb_hydro_idx32(h->ncell);
+    L.map_u0 = stage2 && maps == h->maps ? NB_MAP_RHO : -1;      // stage 2 of a step: u0 is the state
     L.wait_limit = h->wait_limit;
     if (h->stall_test) L.maps = nullptr;
     Prof pf(h, (smax || stage2) ? NB_PROF_STAGE2 : NB_PROF_STAGE1, 1);
@@ -957,7 +958,7 @@ struct nb_batch_s {
     cudaStream_t bs = nullptr;          // the batch's own stream (capturable)
     cudaEvent_t ev_in = nullptr, ev_out = nullptr;
     int solver = 0, limiter = 0, max_stars = 1, grid = 0, ray_group = 1;
-    int idx32 = 1;                      // every instance below 2^31 cells: 32-bit cell offsets
+    int idx32 = 1;                      // 32-bit offsets reach every instance's cells
     NbBatchInst* d_inst = nullptr;
     HydroLaunch* d_L1 = nullptr;
     HydroLaunch* d_L2 = nullptr;
@@ -1006,6 +1007,7 @@ HydroLaunch stage_desc(nb_instance* h, bool stage2) {
     L.sw = h->sw;
     L.maps = h->maps;
     L.map_in = stage2 ? NB_MAP_S0 : NB_MAP_RHO;
+    L.map_u0 = stage2 ? NB_MAP_RHO : -1;
     for (int c = 0; c < 4; ++c) {
         float* S = plane(h, c);
         float* U[4] = {f.rho, f.mx, f.my, f.mz};
@@ -1151,7 +1153,7 @@ NB_EXPORT int nb_batch_create(const nb_handle* hs, const int* ion_every, int n, 
     for (auto* h : b->inst) {
         b->max_stars = std::max(b->max_stars, h->nstars);
         b->n_plane += h->hc.plane_on ? 1 : 0;
-        if (h->ncell >= (1LL << 31)) b->idx32 = 0;
+        if (!nb_hydro_idx32(h->ncell)) b->idx32 = 0;
     }
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);

@@ -108,7 +108,8 @@ struct HydroLaunch {
     int nstars_host;             // == c->nstars (sizes the dynamic shared memory)
     int no_sources;              // stirring-phase hydro: no stars, wind or jets (sim.py:1046)
     int order;                   // tile sweep order (NB_TUNE_TILE_ORDER)
-    int idx32;                   // fewer than 2^31 cells: 32-bit cell offsets (single-instance stage)
+    int idx32;                   // 32-bit offsets reach every cell (nb_hydro_idx32)
+    int map_u0;                  // first of the four maps of u0, whose planes stage 2 prefetches; -1: none
     unsigned wait_limit;         // polls of each bounded TMA wait (NB_TUNE_WAIT_LIMIT)
     int active;                  // batched stage: 0 = the instance's slot is idle (its tiles are skipped)
 };
@@ -220,9 +221,18 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
         : "memory");
 }
 
+// a 3D tile into L2 only (no completion to wait for; c0 a multiple of 4 floats)
+__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap* map, int c0, int c1, int c2) {
+    asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(
+                     reinterpret_cast<uint64_t>(map)),
+                 "r"(c0), "r"(c1), "r"(c2)
+                 : "memory");
+}
+
 // ------------------------------------------------------------------ launchers (nb_*.cu)
 cudaError_t nb_launch_hydro(const HydroLaunch& L, int solver, int limiter, cudaStream_t s);
 int nb_hydro_tile_j();
+int nb_hydro_idx32(long long ncell);     // the stage's 32-bit offsets reach every cell of a grid this large
 // Batches of up to NB_BATCH_PARAM_MAX instances (32-bit cell offsets) hand the persistent stage
 // kernel their stage records as one kernel parameter (28 KB of the 32 KB parameter space): the
 // kernel then reads a record's fields from the constant bank, as the single-instance kernel reads
