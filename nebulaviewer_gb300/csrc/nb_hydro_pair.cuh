@@ -19,9 +19,9 @@
 // of two warps, done a step ahead.  128 registers, 108 KB of shared memory, two blocks per SM.
 //
 // Bound: instruction issue at 16 warps a SM (issue active ~60%; barrier, shared-memory and fixed
-// latencies about equal), not bytes and not one pipe: 300 / 320 thread instructions a cell where pairs
-// of components took 528 / 559.  Measured at 256^3 (sheet, 20-plane chunks): stage 1 309 -> 245 us,
-// stage 2 338 -> 261 us (2.46 and 3.35 TB/s of their 36 and 52 B a cell); 192^3 145 -> 118, 160 -> 125 us.
+// latencies about equal), not bytes and not one pipe: 320 / 340 thread instructions a cell where pairs
+// of components took 528 / 559.  Measured at 256^3 (sheet, 20-plane chunks): stage 1 309 -> 252 us,
+// stage 2 338 -> 271 us (2.40 and 3.22 TB/s of their 36 and 52 B a cell); 192^3 145 -> 121, 160 -> 130 us.
 // Tried on this tile and slower or level: the own cells' values read again from global memory (one
 // address instruction and a pointer load per access, +12%), shuffles along k (+3%), the march unrolled
 // by two (instructions -5%, instruction fetch stalls +), a ninth and tenth warp for the edge work (96
@@ -33,8 +33,7 @@ namespace {
 
 constexpr int HYDRO_TJ = 16;          // tile rows along j (two rows per warp)
 constexpr int HYDRO_THREADS = 256;    // eight warps
-constexpr int PPW = 37;               // pairs per row of a plane: columns k0-2 .. k0+33 and one pad (the edge
-                                      // warp reads down a column: 592-byte rows spread it over all banks)
+constexpr int PPW = 36;               // pairs per row of a plane: columns k0-2 .. k0+33
 constexpr long long HYDRO_IDX32_CELLS = (1LL << 31) - 1;       // signed cell offsets
 constexpr int HYDRO_MINB = 2;         // resident blocks per SM (128 registers, 80 KB of shared memory each)
 constexpr int HYDRO_ROT_STEP = 2;     // two resident blocks place their extra work two schedulers apart
@@ -236,19 +235,20 @@ struct HydroSmem {
     static constexpr int NP = TJ / 2;                                        // row pairs, one per warp
     static constexpr int RAW_FIELD = (TJ + 4) * RAWW * 4;                    // one field of the raw slot
     static constexpr int PLANE = (NP + 2) * PPW * 16;                        // one array over a plane with its halo
-    // a slot: (r0 r1 u0 u1), (v0 v1 w0 w1) and (c2_0 c2_1 c_0 c_1) of every pair, three arrays
-    static constexpr int SLOT = (3 * PLANE + 127) / 128 * 128;
+    // a slot: (r0 r1 u0 u1), (v0 v1 w0 w1) and (c2_0 c2_1 c_0 c_1) of every pair, then the own cells' raw
+    // (rho, mx) and (my, mz), [256] each
+    static constexpr int OWN = 3 * PLANE;
     static constexpr int PER = HYDRO_THREADS * 16;                           // 16 bytes per thread
     static constexpr int RAW = 0;                                            // five fields: plane p as loaded
+    static constexpr int SLOT = OWN + 2 * PER;
     // a warp's exchange along k, [2 halves][256], and beside it the edges [parity][side][NP] of each half:
     // side 0 the z face before the tile, side 1 the lower state of the cell after it
     static constexpr int ZX = (RAW + 5 * RAW_FIELD + 511) / 512 * 512;
     static constexpr int ZE = ZX + PER, ZE_PAR = 256, ZE_SIDE = 128;         // ZE: a multiple of 512
     static constexpr int ZX_HALF = PER + 512;
     static constexpr int FY = ZX + 2 * ZX_HALF;                              // the y face below each pair, [parity][256]
-    static constexpr int OWN = FY + 2 * PER;                                 // the own cells: (r, mx), (my, mz), xi;
-    static constexpr int OWN_X = OWN + 4 * PER;                              // each [parity][256]
-    static constexpr int PRIM = OWN_X + PER;                                 // slots of planes p-2, p-1, p
+    static constexpr int XI = FY + 2 * PER;                                  // the own cells' xi, [parity][256]
+    static constexpr int PRIM = XI + PER;                                    // slots of planes p-2, p-1, p
     static constexpr int BAR_BYTES = 64;
     static constexpr int FIXED = PRIM + 3 * SLOT + BAR_BYTES;
     static constexpr int FLAG = FIXED - BAR_BYTES + 16;                      // after two mbarriers: a wait gave up
@@ -362,15 +362,15 @@ __device__ __forceinline__ void hydro_tile(const HydroLaunch& L, int tile, unsig
     const Idx plane = (Idx)ny * nz, at = (Idx)min(j, ny - 1) * nz + min(k, nz - 1);
     const int up_row = j + 1 < ny ? nz : 0;
 
-    const float a = STAGE2 ? L.a : L.a + L.b, bdt = L.b * dt;         // stage 1: U0 is U
-    const float kdiv = bdt * (C.dx_pow2 ? -C.inv_dx : -1.0f / dx);
+    const float ab = L.a + L.b, bdt = L.b * dt, kdiv = -__fdiv_rn(bdt, dx);
+    const float src = kdiv != 0.0f ? __fdiv_rn(bdt, kdiv) : 0.0f;       // -dx, such that kdiv src is b dt
     float vmax_local = 0.0f;
     St<F2> Lx{}, fxp{}, S{};                         // plane p-1's upper x state; the last x face; plane p-2's y and
     St<float> f1{};                                  // z differences, and its face between the two rows
     F2 u0[4];                                        // stage 2: u0 of the plane the next step updates
     // offsets that a step leaves for the next: the own pair in the slots of planes p, p-1, p-2; the own
     // 16 bytes of the parity of p - P0; where the next lane's lower state and the previous lane's face are
-    const int own = (tj + 1) * ROW + (tk + 2) * 16;
+    const int own = (tj + 1) * ROW + (tk + 2) * 16, raw_place = SM::OWN + tid * 16 - own;
     int o0 = own, o1 = own + 2 * SM::SLOT, o2 = own + SM::SLOT, t0 = tid * 16;
     int z_up = tk == 31 ? SM::ZE + SM::ZE_SIDE + SM::ZE_PAR + tj * 16 : SM::ZX + tid * 16 + 16;
     int z_dn = tk == 0 ? SM::ZE + SM::ZE_PAR + tj * 16 : SM::ZX + tid * 16 - 16;
@@ -383,18 +383,13 @@ __device__ __forceinline__ void hydro_tile(const HydroLaunch& L, int tile, unsig
     auto step = [&](const int p, auto full, auto second) -> bool {
         constexpr bool FULL = decltype(full)::value, SEC = decltype(second)::value;   // SEC: plane P0+1
         constexpr int RAW = SEC ? SECOND : SM::RAW;
-        // the own cells of plane i = p - 2, which the update needs: the Runge-Kutta combination
-        // a U0 + b (U + dt dU) without its flux term
         const int i = p - 2;
-        F2 base[4];
-        if (FULL) {
-            const St<F2> u = state(SM::OWN + t0, 2 * SM::PER);
-            const float2 x = *reinterpret_cast<const float2*>(smem + SM::OWN_X + (t0 >> 1));
-            base[0] = u.r; base[1] = u.n; base[2] = u.s; base[3] = u.t;
-#pragma unroll
-            for (int f = 0; f < 4; ++f)
-                base[f] = STAGE2 ? vfma(vset<F2>(a), u0[f], vmul(vset<F2>(L.b), base[f])) : vmul(vset<F2>(a), base[f]);
-            // ---- wind and jets (nebula3d.py:111-149)
+        if (FULL && (wind > 0.0f || n_jet > 0)) {
+            // ---- wind and jets of plane i (nebula3d.py:111-149), into its flux differences, which
+            // the update scales by kdiv
+            const float4 u = ld4(SM::PRIM + o2 + raw_place);
+            const float2 x = *reinterpret_cast<const float2*>(smem + SM::XI + (t0 >> 1));
+            const F2 rho = vmul(vset<F2>(src), mk2(u.x, u.y));
             const float px = ((float)i + 0.5f) * dx, py0 = ((float)j + 0.5f) * dx, py1 = ((float)(j + 1) + 0.5f) * dx;
             const float pz = ((float)k + 0.5f) * dx;
             if (wind > 0.0f && (x.x > 0.01f || x.y > 0.01f)) {
@@ -412,11 +407,11 @@ __device__ __forceinline__ void hydro_tile(const HydroLaunch& L, int tile, unsig
                     }
                 }
                 // cells at or below an ionized fraction of 0.01 take no wind
-                const float w = wind * bdt;
-                const F2 wx = vmul(u.r, mk2(x.x > 0.01f ? w * x.x : 0.0f, x.y > 0.01f ? w * x.y : 0.0f));
-                base[1] = vfma(wx, ax, base[1]);
-                base[2] = vfma(wx, ay, base[2]);
-                base[3] = vfma(wx, az, base[3]);
+                // cells at or below an ionized fraction of 0.01 take no wind
+                const F2 wx = vmul(rho, mk2(x.x > 0.01f ? wind * x.x : 0.0f, x.y > 0.01f ? wind * x.y : 0.0f));
+                S.n = vfma(wx, ax, S.n);
+                S.s = vfma(wx, ay, S.s);
+                S.t = vfma(wx, az, S.t);
             }
             if (n_jet > 0) {
                 float jx[2] = {0.0f, 0.0f}, jy[2] = {0.0f, 0.0f}, jz[2] = {0.0f, 0.0f};
@@ -436,10 +431,9 @@ __device__ __forceinline__ void hydro_tile(const HydroLaunch& L, int tile, unsig
                         }
                     }
                 }
-                const F2 rb = vmul(u.r, vset<F2>(bdt));
-                base[1] = vfma(rb, mk2(jx[0], jx[1]), base[1]);
-                base[2] = vfma(rb, mk2(jy[0], jy[1]), base[2]);
-                base[3] = vfma(rb, mk2(jz[0], jz[1]), base[3]);
+                S.n = vfma(rho, mk2(jx[0], jx[1]), S.n);
+                S.s = vfma(rho, mk2(jy[0], jy[1]), S.s);
+                S.t = vfma(rho, mk2(jz[0], jz[1]), S.t);
             }
         }
         const bool ok = mbar_wait_limited(&bar[SEC ? 1 : 0], SEC ? ph0 >> 1 : ph0 & 1u, &L.wait_limit);
@@ -452,9 +446,9 @@ __device__ __forceinline__ void hydro_tile(const HydroLaunch& L, int tile, unsig
             };
             const F2 w0 = rd(0), w1 = rd(1), w2 = rd(2), w3 = rd(3), x = rd(4);
             if (decltype(own_cells)::value) {
-                st4(SM::OWN + t0, w0, w1);
-                st4(SM::OWN + 2 * SM::PER + t0, w2, w3);
-                *reinterpret_cast<float2*>(smem + SM::OWN_X + (t0 >> 1)) = make_float2(lo(x), hi(x));
+                st4(SM::PRIM + o + raw_place, w0, w1);
+                st4(SM::PRIM + o + raw_place + SM::PER, w2, w3);
+                *reinterpret_cast<float2*>(smem + SM::XI + (t0 >> 1)) = make_float2(lo(x), hi(x));
             }
             const F2 r = vmax(w0, floor_), ri = vrcp(r);
             const St<F2> q = {r, vmul(w1, ri), vmul(w2, ri), vmul(w3, ri)};
@@ -498,9 +492,18 @@ __device__ __forceinline__ void hydro_tile(const HydroLaunch& L, int tile, unsig
             S.n = mk2(lo(S.n) + (f1.n - fm.y), hi(S.n));
             S.s = mk2(lo(S.s) + (f1.s - fm.z), hi(S.s));
             S.t = mk2(lo(S.t) + (f1.t - fm.w), hi(S.t));
-            const F2 kd = vset<F2>(kdiv);
-            const F2 o[4] = {vfma(kd, vadd(vsub(fx.r, fxp.r), S.r), base[0]), vfma(kd, vadd(vsub(fx.n, fxp.n), S.n), base[1]),
-                             vfma(kd, vadd(vsub(fx.s, fxp.s), S.s), base[2]), vfma(kd, vadd(vsub(fx.t, fxp.t), S.t), base[3])};
+            // a U0 + b (U + dt dU) as (a + b) U + (a (U0 - U) + b dt dU): U0 - U is small beside U, so the sum
+            // is rounded once at U's size (in stage 1 U0 is U).  The density's error against float64 after three
+            // steps is 0.8 times that of the sum as written; a U0 + b U formed a step early, which keeps 8
+            // registers free and is 4% faster, makes it 1.15 times
+            const St<F2> u = state(SM::PRIM + o2 + raw_place, SM::PER);
+            const F2 kd = vset<F2>(kdiv), ab2 = vset<F2>(ab), a2 = vset<F2>(L.a);
+            auto comb = [&](F2 fn, F2 fo, F2 sd, F2 un, F2 uo) {
+                const F2 dv = vadd(vsub(fn, fo), sd);
+                return STAGE2 ? vfma(ab2, un, vfma(kd, dv, vmul(a2, vsub(uo, un)))) : vfma(kd, dv, vmul(ab2, un));
+            };
+            const F2 o[4] = {comb(fx.r, fxp.r, S.r, u.r, u0[0]), comb(fx.n, fxp.n, S.n, u.n, u0[1]),
+                             comb(fx.s, fxp.s, S.s, u.s, u0[2]), comb(fx.t, fxp.t, S.t, u.t, u0[3])};
             fxp = fx;
             const F2 r = vmax(o[0], floor_);
             // one reciprocal for the three velocities and the max speed; the speed cap without a branch
