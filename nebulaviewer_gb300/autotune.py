@@ -93,7 +93,9 @@ def autotune(sim, knobs=None, steps=4, use_cache=True):
     try:
         for knob in knobs:
             best = None
-            for v in CANDIDATES[knob]:
+            # the library's own choice of the depth competes with the fixed ones
+            extra = (orig[knob],) if knob == "chunk_i" and orig[knob] not in CANDIDATES[knob] else ()
+            for v in CANDIDATES[knob] + extra:
                 put(sim, knob, v)
                 restore()
                 _measure(sim, knob, 1)                 # warm the launch path

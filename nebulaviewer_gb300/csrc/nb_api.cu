@@ -37,7 +37,8 @@ struct nb_instance {
     int nstars = 0, star_alloc = 0;
     long long host_it = 0;
     int smax_valid = 0;
-    int chunk_i = 20, ray_group = 1, fuv_group = 16;      // measured best at 192^3-256^3 (nb_set_tuning)
+    int chunk_i = 20, chunk_set = 0;    // planes per hydro tile, chosen for the grid (nb_create) or set (nb_set_tuning)
+    int ray_group = 1, fuv_group = 16;  // measured best at 192^3-256^3 (nb_set_tuning)
     int tile_order = 0;
     int front_cull = 1;                 // apply_front skips the stars that cannot change a segment
     int fuv_cut = 1;                    // FUV rays stop where exp(-tau) has reached 0.0f
@@ -145,6 +146,22 @@ bool is_pow2(double x) {
 int upload_const(nb_instance* h) {
     CK(h, cudaMemcpyAsync(h->c, &h->hc, sizeof(NbConst), cudaMemcpyHostToDevice, h->stream));
     return NB_OK;
+}
+
+int sm_count() {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+        cudaGetLastError();                      // no device: nb_create reports it at its first allocation
+        sms = 0;
+    }
+    return sms > 0 ? sms : 152;
+}
+
+// (k, j) tile columns of a grid
+long long hydro_columns(const nb_desc& d) {
+    const int tj = nb_hydro_tile_j();
+    return (long long)((d.nz + 31) / 32) * ((d.ny + tj - 1) / tj);
 }
 
 float* plane(nb_instance* h, int p) { return h->d.f.stage + (long long)p * h->ncell; }
@@ -326,6 +343,7 @@ NB_EXPORT int nb_create(const nb_desc* d, nb_handle* out) {
         delete h;
         return fail(nullptr, NB_ERR_LIMIT, "grid too large (ny * nz and fnu * fnphi * fnr must stay below 2^31)");
     }
+    h->chunk_i = nb_hydro_depth(d->nx, hydro_columns(*d), sm_count());
     NbConst& c = h->hc;
     c.nx = d->nx; c.ny = d->ny; c.nz = d->nz; c.nstars = 0;
     c.dx_pow2 = is_pow2(d->dx) ? 1 : 0;
@@ -907,6 +925,7 @@ NB_EXPORT int nb_set_tuning(nb_handle h, int key, int value) {
         case NB_TUNE_CHUNK_I:
             if (value < 1) return fail(h, NB_ERR_ARG, "chunk_i must be >= 1");
             h->chunk_i = value;
+            h->chunk_set = 1;
             return NB_OK;
         case NB_TUNE_TILE_ORDER:
             if (value != 0 && value != 1) return fail(h, NB_ERR_ARG, "tile order must be 0 or 1");
@@ -999,7 +1018,8 @@ int bfail(nb_batch_s* b, int code, const std::string& m) {
         if (e_ != cudaSuccess) return bfail((b), NB_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
     } while (0)
 
-HydroLaunch stage_desc(nb_instance* h, bool stage2) {
+// `depth`: planes per tile where none was set for the instance
+HydroLaunch stage_desc(nb_instance* h, bool stage2, int depth) {
     HydroLaunch L{};
     const nb_fields& f = h->d.f;
     L.c = h->c;
@@ -1023,7 +1043,8 @@ HydroLaunch stage_desc(nb_instance* h, bool stage2) {
     const int tj = nb_hydro_tile_j();
     L.tiles_k = (h->d.nz + 31) / 32;
     L.tiles_j = (h->d.ny + tj - 1) / tj;
-    L.chunk_i = h->chunk_i < h->d.nx ? h->chunk_i : h->d.nx;
+    const int chunk = h->chunk_set ? h->chunk_i : depth;
+    L.chunk_i = chunk < h->d.nx ? chunk : h->d.nx;
     L.n_chunks = (h->d.nx + L.chunk_i - 1) / L.chunk_i;
     L.nstars_host = h->nstars;
     L.order = h->tile_order;
@@ -1155,11 +1176,8 @@ NB_EXPORT int nb_batch_create(const nb_handle* hs, const int* ion_every, int n, 
         b->n_plane += h->hc.plane_on ? 1 : 0;
         if (!nb_hydro_idx32(h->ncell)) b->idx32 = 0;
     }
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int params = b->idx32 && n <= NB_BATCH_PARAM_MAX;
-    b->grid = (sms > 0 ? sms : 152) * nb_hydro_batch_blocks_per_sm(b->solver, b->limiter, b->max_stars, b->idx32, params);
+    b->grid = sm_count() * nb_hydro_batch_blocks_per_sm(b->solver, b->limiter, b->max_stars, b->idx32, params);
     if (cudaStreamCreateWithFlags(&b->bs, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&b->ev_in, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&b->ev_out, cudaEventDisableTiming) != cudaSuccess)
@@ -1173,11 +1191,14 @@ NB_EXPORT int nb_batch_create(const nb_handle* hs, const int* ion_every, int n, 
     L2.resize(n);
     b->active.assign(n, 1);
     b->n_active = n;
+    double planes = 0.0;
+    for (auto* h : b->inst) planes += (double)hydro_columns(h->d) * h->d.nx;
+    const int depth = nb_hydro_depth_batch(planes, b->grid);
     for (int i = 0; i < n; ++i) {
         nb_instance* h = b->inst[i];
         bi[i] = NbBatchInst{h->c, h->st, h->stars, h->sw, h->nstars, 1};
-        L1[i] = stage_desc(h, false);
-        L2[i] = stage_desc(h, true);
+        L1[i] = stage_desc(h, false, depth);
+        L2[i] = stage_desc(h, true, depth);
     }
     if (params) {                                // the records as the persistent kernel's parameter
         b->rec1.reset(new NbBatchRecords());

@@ -18,6 +18,7 @@
 // Sources: the wind loop over the active stars in ionized cells, the jet loop over the tile's list
 // of stars whose jet can reach it.  Stage 2 also reduces the CFL max speed of the new state
 // (nebula3d.py:154-162) into one atomic.
+#include <cmath>
 #include <type_traits>
 
 #include "nb_internal.cuh"
@@ -290,6 +291,39 @@ cudaError_t run_batch(const HydroLaunch* Ls, const NbBatchRecords* rec, const in
 }  // namespace
 
 int nb_hydro_tile_j() { return HYDRO_TJ; }
+
+// The i-chunk depth of a stage alone on the GPU: blocks = columns x chunks run in rounds of `sms` x
+// HYDRO_MINB, each of the depth's planes and four halo planes (and about half a plane to start); a
+// last round with fewer blocks on an SM has cheaper planes.  The least time over all chunk counts.
+// With a fixed depth of 20 a small grid left SMs idle for 24 serial planes and the last round was
+// often nearly empty: stages 1 + 2 (fast) at 64^3 76 -> 33 us, 128^3 96 -> 88, 192^3 251 -> 235,
+// 256^3 523 -> 502 (depths 4, 15, 48, 37).
+int nb_hydro_depth(int nx, long long columns, int sms) {
+    int best = nx;
+    double least = 0.0;
+    for (int n = 1, last = 0; n <= nx; ++n) {
+        const int depth = (nx + n - 1) / n;
+        if (depth == last) continue;                       // the same depth with fewer chunks came before
+        last = depth;
+        const long long blocks = columns * ((nx + depth - 1) / depth), round = (long long)sms * HYDRO_MINB;
+        const long long rest = blocks % round;
+        const double t = ((double)(blocks / round) + HYDRO_PLANE[(rest + sms - 1) / sms]) * (depth + 4.5);
+        if (least == 0.0 || t < least) {
+            least = t;
+            best = depth;
+        }
+        if (depth == 1) break;
+    }
+    return best;
+}
+
+// The depth of a batch's stages, whose persistent blocks (`slots` of them) take tiles in turn: deep
+// chunks convert fewer halo planes (4.5 per chunk), shallow ones end together (half a chunk idle at the
+// end); the sum is least at the depth whose square is 9 planes' worth of each block's share.
+int nb_hydro_depth_batch(double column_planes, int slots) {
+    const double d = std::sqrt(9.0 * column_planes / (slots > 0 ? slots : 1));
+    return d < 2.0 ? 2 : (d > 128.0 ? 128 : (int)d);
+}
 
 int nb_hydro_idx32(long long ncell) { return ncell <= HYDRO_IDX32_CELLS; }
 
