@@ -30,7 +30,7 @@ struct nb_instance {
     float* scratch3 = nullptr;          // 3 floats: a single star position for the one-star kernels
     float* plane_xf = nullptr;          // [ny][nz] front of the -x plane source
     double* red = nullptr;              // FP64 reduction partials
-    float2* front_parts = nullptr;      // per-star front-radius ranges (apply_front)
+    uint2* front_bounds = nullptr;      // per-star front-radius ranges (apply_front)
     float* drive_ring = nullptr;        // stirring fields [slots][3][sx][sy][sz]
     NbState* state_mirror = nullptr;    // pinned host copy of the control block (nb_mirror_clock, nb_set_clock)
     long long drive_field = 0;          // floats per forcing field (3 components)
@@ -209,12 +209,14 @@ int do_ionize(nb_instance* h) {
     const nb_fields& f = h->d.f;
     {
         Prof pf(h, NB_PROF_CTRL, 1);
-        CK(h, nb_launch_weights(h->c, h->st, h->stars, h->sw, h->nstars, h->stream));
+        CK(h, nb_launch_weights(h->c, h->st, h->stars, h->sw, h->nstars, h->front_bounds, h->stream));
     }
+    const bool cull = h->front_cull && h->nstars >= 1 && h->nstars <= NB_ROW_STARS;
     if (h->nstars > 0) {
         Prof pf(h, NB_PROF_CAST_RAYS, 1);
-        CK(h, nb_launch_cast_rays(h->c, h->sw, h->dirs, f.rho, h->rfront, h->nstars, h->ray_group, nullptr, 0.0f,
-                                  h->stream, h->d.nu, h->d.nphi, h->front_pairs));
+        CK(h, nb_launch_cast_rays(h->c, h->sw, h->dirs, f.rho, h->rfront, h->nstars, h->ray_group,
+                                  cull ? h->front_bounds : nullptr, nullptr, 0.0f, h->stream, h->d.nu, h->d.nphi,
+                                  h->front_pairs, h->ncell < (1LL << 31)));
     }
     if (h->hc.plane_on) {
         Prof pf(h, NB_PROF_CAST_RAYS, 1);
@@ -222,12 +224,10 @@ int do_ionize(nb_instance* h) {
     }
     float* xi_raw = plane(h, 0);            // sim.py:928-941: xi_tmp lives in the stage block
     {
-        const bool cull = h->front_cull && h->nstars >= 1 && h->nstars <= NB_ROW_STARS;
-        Prof pf(h, NB_PROF_APPLY_FRONT, cull ? 2 : 1);
+        Prof pf(h, NB_PROF_APPLY_FRONT, 1);
         CK(h, nb_launch_apply_front(h->c, h->sw, h->rfront, h->nstars, xi_raw, f.dfront, &h->st->smax_bits,
                                     h->stream, h->d.nx, h->d.ny, h->d.fields_fp32 ? 0 : 1,
-                                    cull ? h->front_parts : nullptr,
-                                    (long long)h->d.nu * h->d.nphi, h->front_pairs));
+                                    cull ? h->front_bounds : nullptr, h->front_pairs));
     }
     {
         Prof pf(h, NB_PROF_SMOOTH, 1);
@@ -390,7 +390,7 @@ NB_EXPORT int nb_create(const nb_desc* d, nb_handle* out) {
     c.plane_xf = h->plane_xf;
     c.plane_g0 = f.stage + 2 * h->ncell;
     CKC(cudaMalloc(&h->red, sizeof(double) * nb_reduce_scratch_doubles()));
-    CKC(cudaMalloc(&h->front_parts, sizeof(float2) * NB_ROW_STARS * NB_FRONT_PARTS));
+    CKC(cudaMalloc(&h->front_bounds, sizeof(uint2) * NB_ROW_STARS));
     CKC(cudaMallocHost(&h->state_mirror, sizeof(NbState)));
     std::memset(h->state_mirror, 0, sizeof(NbState));
     CKC(cudaMemsetAsync(h->st, 0, sizeof(NbState), h->stream));
@@ -425,7 +425,7 @@ static long long instance_bytes(const nb_desc& d, long long star_alloc, long lon
     b += (long long)sizeof(float4) * ((long long)d.nu * d.nphi + (long long)d.fnu * d.fnphi);
     b += 4 * sizeof(float) + sizeof(float) * ncell_plane;
     b += (long long)sizeof(double) * nb_reduce_scratch_doubles();
-    b += (long long)sizeof(float2) * NB_ROW_STARS * NB_FRONT_PARTS;
+    b += (long long)sizeof(uint2) * NB_ROW_STARS;
     b += 2LL * sizeof(float) * star_alloc * ((long long)d.nu * d.nphi + (long long)d.fnr * d.fnu * d.fnphi);
     return b + ring_bytes;
 }
@@ -446,7 +446,7 @@ NB_EXPORT void nb_destroy(nb_handle h) {
     if (h->stream) cudaStreamSynchronize(h->stream);
     else cudaDeviceSynchronize();
     void* ps[] = {h->c, h->st, h->stars, h->sw, h->maps, h->tmp_maps, h->dirs, h->dirs_fuv,
-                  h->rfront, h->att, h->scratch3, h->red, h->plane_xf, h->drive_ring, h->front_parts};
+                  h->rfront, h->att, h->scratch3, h->red, h->plane_xf, h->drive_ring, h->front_bounds};
     for (void* p : ps)
         if (p) cudaFree(p);
     if (h->state_mirror) cudaFreeHost(h->state_mirror);
@@ -752,7 +752,7 @@ NB_EXPORT int nb_fuv(nb_handle h) {
     }
     {
         Prof pf(h, NB_PROF_CTRL, 1);
-        CK(h, nb_launch_weights(h->c, h->st, h->stars, h->sw, h->nstars, h->stream));
+        CK(h, nb_launch_weights(h->c, h->st, h->stars, h->sw, h->nstars, nullptr, h->stream));
     }
     if (h->nstars > 0) {
         Prof pf(h, NB_PROF_CAST_FUV, 2);                // the (rho, xi) pack into stage planes 0-1 + the rays
@@ -783,7 +783,7 @@ NB_EXPORT int nb_hydro_stage(nb_handle h, const float* const in4[4], const float
         if (!encode_plane(&hm[f], in4[f], h->d.nx, h->d.ny, h->d.nz)) return fail(h, NB_ERR_CUDA, "tensor map");
     if (!encode_plane(&hm[NB_MAP_XI], h->d.f.xi, h->d.nx, h->d.ny, h->d.nz)) return fail(h, NB_ERR_CUDA, "tensor map");
     CK(h, cudaMemcpyAsync(h->tmp_maps, hm, sizeof(CUtensorMap) * 5, cudaMemcpyHostToDevice, h->stream));
-    CK(h, nb_launch_weights(h->c, h->st, h->stars, h->sw, h->nstars, h->stream));
+    CK(h, nb_launch_weights(h->c, h->st, h->stars, h->sw, h->nstars, nullptr, h->stream));
     int rc = launch_stage(h, in4, u0_4, out4, 0, h->tmp_maps, a, b, true, dt, pulse, false);
     if (rc != NB_OK) return rc;
     CK(h, cudaStreamSynchronize(h->stream));        // tmp_maps is reused by the next call
@@ -806,8 +806,8 @@ NB_EXPORT int nb_cast_rays(nb_handle h, const double xyz[3], double Q, float* rf
     if (!h || !xyz || !rfront_out) return fail(h, NB_ERR_ARG, "null argument");
     float s3[4] = {(float)xyz[0], (float)xyz[1], (float)xyz[2], 0.f};
     CK(h, cudaMemcpyAsync(h->scratch3, s3, sizeof(s3), cudaMemcpyHostToDevice, h->stream));
-    CK(h, nb_launch_cast_rays(h->c, h->sw, h->dirs, h->d.f.rho, rfront_out, 1, h->ray_group, h->scratch3, (float)Q,
-                              h->stream, h->d.nu, h->d.nphi, 0));
+    CK(h, nb_launch_cast_rays(h->c, h->sw, h->dirs, h->d.f.rho, rfront_out, 1, h->ray_group, nullptr, h->scratch3,
+                              (float)Q, h->stream, h->d.nu, h->d.nphi, 0, h->ncell < (1LL << 31)));
     CK(h, cudaStreamSynchronize(h->stream));
     return NB_OK;
 }
@@ -977,6 +977,7 @@ struct nb_batch_s {
     cudaStream_t bs = nullptr;          // the batch's own stream (capturable)
     cudaEvent_t ev_in = nullptr, ev_out = nullptr;
     int solver = 0, limiter = 0, max_stars = 1, grid = 0, ray_group = 1;
+    int small = 1;                      // every instance below 2^31 cells (the ray cast's 32-bit indices)
     int idx32 = 1;                      // 32-bit offsets reach every instance's cells
     NbBatchInst* d_inst = nullptr;
     HydroLaunch* d_L1 = nullptr;
@@ -1071,7 +1072,7 @@ NbRayJob ray_job(nb_instance* h) {
     J.smax = &h->st->smax_bits;
     J.nstars = h->nstars;
     J.half = h->d.fields_fp32 ? 0 : 1;
-    J.front_parts = (h->front_cull && h->nstars >= 1 && h->nstars <= NB_ROW_STARS) ? h->front_parts : nullptr;
+    J.front_bounds = (h->front_cull && h->nstars >= 1 && h->nstars <= NB_ROW_STARS) ? h->front_bounds : nullptr;
     J.nray = (long long)h->d.nu * h->d.nphi;
     J.pairs = h->front_pairs;
     J.active = 1;
@@ -1102,7 +1103,7 @@ int batch_hydro(nb_batch_s* b) {
 
 int batch_ionize(nb_batch_s* b, const NbRayJob* jobs, const NbRayJob* host_jobs, int n_jobs, long long groups,
                  long long blocks, const std::vector<int>& listed) {
-    b->launches += 5;                       // control, rays, front ranges, front apply, smoothing
+    b->launches += 4;                       // control, rays, front apply, smoothing
     BCK(b, nb_launch_ctrl_batch(b->d_inst, (int)b->inst.size(), 0, nullptr, b->bs));
     for (int i : listed) {
         nb_instance* h = b->inst[i];
@@ -1110,7 +1111,7 @@ int batch_ionize(nb_batch_s* b, const NbRayJob* jobs, const NbRayJob* host_jobs,
         b->launches += 1;
         BCK(b, nb_launch_plane_front(h->c, h->d.f.rho, h->plane_xf, h->d.ny, h->d.nz, b->bs));
     }
-    BCK(b, nb_launch_ionize_batch(jobs, host_jobs, n_jobs, groups, blocks, b->ray_group, b->bs));
+    BCK(b, nb_launch_ionize_batch(jobs, host_jobs, n_jobs, groups, blocks, b->ray_group, b->small, b->bs));
     return NB_OK;
 }
 
@@ -1131,9 +1132,9 @@ int batch_run_graph(nb_batch_s* b, cudaGraphExec_t* g, int ion) {
         e = cudaGraphInstantiate(g, graph, 0);
         cudaGraphDestroy(graph);
         if (e != cudaSuccess) return bfail(b, NB_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
-        b->launches -= ion ? 8 + b->n_plane : 3;       // captured, not launched
+        b->launches -= ion ? 7 + b->n_plane : 3;       // captured, not launched
     }
-    b->launches += ion ? 8 + b->n_plane : 3;
+    b->launches += ion ? 7 + b->n_plane : 3;
     BCK(b, cudaGraphLaunch(*g, b->bs));
     return NB_OK;
 }
@@ -1175,6 +1176,7 @@ NB_EXPORT int nb_batch_create(const nb_handle* hs, const int* ion_every, int n, 
         b->max_stars = std::max(b->max_stars, h->nstars);
         b->n_plane += h->hc.plane_on ? 1 : 0;
         if (!nb_hydro_idx32(h->ncell)) b->idx32 = 0;
+        if (h->ncell >= (1LL << 31)) b->small = 0;
     }
     const int params = b->idx32 && n <= NB_BATCH_PARAM_MAX;
     b->grid = sm_count() * nb_hydro_batch_blocks_per_sm(b->solver, b->limiter, b->max_stars, b->idx32, params);
@@ -1196,7 +1198,7 @@ NB_EXPORT int nb_batch_create(const nb_handle* hs, const int* ion_every, int n, 
     const int depth = nb_hydro_depth_batch(planes, b->grid);
     for (int i = 0; i < n; ++i) {
         nb_instance* h = b->inst[i];
-        bi[i] = NbBatchInst{h->c, h->st, h->stars, h->sw, h->nstars, 1};
+        bi[i] = NbBatchInst{h->c, h->st, h->stars, h->sw, h->nstars, 1, h->front_bounds};
         L1[i] = stage_desc(h, false, depth);
         L2[i] = stage_desc(h, true, depth);
     }

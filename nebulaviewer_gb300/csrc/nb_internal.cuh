@@ -7,7 +7,6 @@
 
 #include "../../include/nebula.h"
 
-#define NB_FRONT_PARTS 32         // partial front-radius ranges per star (apply_front culling)
 #define NB_ROW_STARS 32           // stars a per-row table holds (more: per-cell form)
 #define NB_MAX_STARS 256          // star-table capacity limit (smem-resident in the kernels)
 #define NB_WAIT_LIMIT (1u << 22)  // iteration cap of every device-side spin wait
@@ -122,6 +121,7 @@ struct NbBatchInst {
     NbStarW* sw;
     int nstars;
     int active;           // 0: an idle slot of the batch (no weights, no clock advance)
+    uint2* bounds;        // the instance's front-radius ranges, reset before an ionization
 };
 
 // One instance of a batched ionization (nebula3d.py:247-315 over many instances in 3 launches).
@@ -142,7 +142,7 @@ struct NbRayJob {
     long long blk0;       // first row block of this job (8 rows per block)
     int nstars;
     int half;
-    float2* front_parts;  // the instance's front-radius partials when apply_front culls, else null
+    uint2* front_bounds;  // the instance's front-radius ranges when apply_front culls, else null
     long long nray;       // rays per star (nu * nphi)
     int pairs;            // the front table holds (u, u + 1) pairs (NB_TUNE_FRONT_PAIRS)
     int active;           // 0: an idle slot of the batch (its rays, fronts and smoothing are skipped)
@@ -254,8 +254,9 @@ cudaError_t nb_launch_hydro_batch(const HydroLaunch* Ls, const NbBatchRecords* r
 cudaError_t nb_launch_ctrl(const NbConst* c, NbState* st, const NbStarDev* stars, NbStarW* sw, int nstars,
                            int advance, cudaStream_t s);
 cudaError_t nb_launch_ctrl_batch(const NbBatchInst* insts, int n, int advance, unsigned* counters, cudaStream_t s);
+// star weights only; bounds (or null): the front-radius ranges to reset
 cudaError_t nb_launch_weights(const NbConst* c, const NbState* st, const NbStarDev* stars, NbStarW* sw,
-                              int nstars, cudaStream_t s);
+                              int nstars, uint2* bounds, cudaStream_t s);
 cudaError_t nb_launch_max_speed(const NbConst* c, const float* rho, const float* mx, const float* my,
                                 const float* mz, const float* xi, unsigned* smax_bits, long n, cudaStream_t s);
 cudaError_t nb_launch_drive(const NbConst* c, const NbState* st, const float* rho, float* mx, float* my, float* mz,
@@ -274,16 +275,16 @@ cudaError_t nb_launch_render_pack(const NbConst* c, const float* rho, const floa
                                   int ny, cudaStream_t s);
 cudaError_t nb_launch_ray_dirs(int nu, int nphi, float4* dirs, cudaStream_t s);
 // pairs: the instance's front table holds (rf(u), rf(u + 1)) float2 pairs (2 * nu * nphi floats per
-// star); a star_override launch writes the reference layout [u][phi] (pairs = 0)
+// star); a star_override launch writes the reference layout [u][phi] (pairs = 0); small: fewer than
+// 2^31 cells
 cudaError_t nb_launch_cast_rays(const NbConst* c, const NbStarW* sw, const float4* dirs, const float* rho,
-                                float* rfront, int nstars, int group, const float* star_override, float q_override,
-                                cudaStream_t s, int nu, int nphi, int pairs);
-// with front_parts (NB_ROW_STARS * NB_FRONT_PARTS float2 scratch) and 1 <= nstars <= NB_ROW_STARS:
-// first each star's front-radius range (one more launch), then segments skip the stars that
-// cannot change them
+                                float* rfront, int nstars, int group, uint2* bounds, const float* star_override,
+                                float q_override, cudaStream_t s, int nu, int nphi, int pairs, int small);
+// bounds: each star's front-radius range, reset by nb_launch_weights and merged by the ray cast (or
+// null); with it and 1 <= nstars <= NB_ROW_STARS segments skip the stars that cannot change them
 cudaError_t nb_launch_apply_front(const NbConst* c, const NbStarW* sw, const float* rfront, int nstars,
                                   float* xi_raw, void* dfront, unsigned* smax_reset, cudaStream_t s, int nx, int ny,
-                                  int half, float2* front_parts, long long nray, int pairs);
+                                  int half, const uint2* bounds, int pairs);
 cudaError_t nb_launch_smooth(const NbConst* c, const float* xi_raw, float* xi, const float* rho, const float* mx,
                              const float* my, const float* mz, unsigned* smax_bits, cudaStream_t s, int nx, int ny);
 // The ray cast of a batch of at most NB_BATCH_PARAM_MAX jobs takes the job records as one kernel
@@ -293,7 +294,7 @@ struct NbRayJobs {
     NbRayJob J[NB_BATCH_PARAM_MAX];
 };
 cudaError_t nb_launch_ionize_batch(const NbRayJob* jobs, const NbRayJob* host_jobs, int n_jobs, long long n_groups,
-                                   long long n_blocks, int group, cudaStream_t s);
+                                   long long n_blocks, int group, int small, cudaStream_t s);
 cudaError_t nb_launch_plane_front(const NbConst* c, const float* rho, float* xf, int ny, int nz, cudaStream_t s);
 cudaError_t nb_launch_plane_fuv(const NbConst* c, const float* rho, const float* xi, float* g, int ny, int nz,
                                 cudaStream_t s);

@@ -6,19 +6,18 @@
 // GB300 design:
 //  * cast_rays: a group of G lanes (1 to 32; 1 by default) marches one ray, G consecutive
 //    samples at a time; the recombination column sum(n^2 r^2 dr) is added to a Kahan-compensated
-//    carry (G > 1: an inclusive group scan; two lanes take it from one exchange; one lane needs
-//    none, which made it the fastest shape once the shuffles' latency led the stalls), and the
-//    first sample whose column passes Q is found with one ballot.  The march is warp-uniform: a
-//    warp's groups loop together until all are done, and the trilinear sampler has no branches,
-//    so the lanes never diverge (divergent exits had made branch resolution the leading stall).
-//    All rays of all active stars are one launch.
+//    carry (G > 1: an inclusive group scan; two lanes take it from one exchange), and the
+//    first sample whose column passes Q is found with one ballot.  That march is warp-uniform: a
+//    warp's groups loop together until all are done, and the trilinear sampler has no branches.
+//    The fast build's one-lane march (cast_ray1) is a plain loop of its own.
+//    All rays of all active stars are one launch, a warp a bundle of neighbouring directions.
 //  * The front table holds, per (star, phi, u), the pair (rf(u), rf(min(u + 1, nu - 1))) as one
 //    float2 (cast_rays writes each front into its own pair and its lower neighbour's), so the
 //    bilinear lookup of apply_front is two 8-byte gathers instead of four 4-byte ones; the values
 //    and the arithmetic are those of the plain table (NB_TUNE_FRONT_PAIRS = 0), bit for bit.
 //  * apply_front: one pass over the grid merges the active stars, in star order, into one
 //    register pair per cell (the reference makes S passes).  With up to 32 stars, each star's
-//    front-radius range (front_bounds_kernel) lets a 32-cell row segment leave out the stars that
+//    front-radius range (merged by the ray cast) lets a 32-cell row segment leave out the stars that
 //    cannot change its xi or front distance (the same bits).  The float32 front distance is
 //    rounded once to the fp16 dfront (sim.py:980-985, 511-514).
 //  * smooth_xi writes the final xi and reduces the CFL max speed of the step from it
@@ -26,6 +25,12 @@
 #include <cstring>
 
 #include "nb_rayutil.cuh"
+#if defined(NB_ARITH_FAST) && NB_ARITH_FAST
+#include "nb_f32x2.cuh"
+#define NB_RAYS_SMALL true         // the fast build's one-lane march on grids of fewer than 2^31 cells
+#else
+#define NB_RAYS_SMALL false
+#endif
 
 namespace {
 
@@ -43,13 +48,11 @@ __global__ void ray_dirs_kernel(int nu, int nphi, float4* __restrict__ dirs) {
     dirs[id] = make_float4(s * cph, s * sph, u, 0.0f);
 }
 
-// nebula3d.py:247-270 cast_rays: ray `ray` of star (sx, sy, sz, Q), G lanes per ray.  `out` is where
-// the front radius goes (a float pointer, 4-byte aligned) with two flags in its low bits: bit 0 also
-// writes out[-1] and bit 1 out[1] (the pair layout's neighbour copies, front_slot); one 64-bit
-// value stays live across the march, as a plain pointer would.
+// nebula3d.py:247-270 cast_rays: ray `ray` of star (sx, sy, sz, Q), G lanes per ray; every
+// lane of the group gets the front radius.
 template <int G>
-__device__ __forceinline__ void cast_ray(const NbConst& C, const float4* __restrict__ dirs,
-                                         const float* __restrict__ rho, uintptr_t out, int ray, float sx, float sy,
+__device__ __forceinline__ float cast_ray(const NbConst& C, const float4* __restrict__ dirs,
+                                         const float* __restrict__ rho, int ray, float sx, float sy,
                                          float sz, float Q, int lane, unsigned gmask, bool live) {
     // Warp-uniform march: every lane of the warp runs the loop until all of its groups are done
     // (`live` false: the group has no ray; `ray` is then any valid index), a finished group's lanes
@@ -127,63 +130,222 @@ __device__ __forceinline__ void cast_ray(const NbConst& C, const float4* __restr
             }
         }
     }
-    if (live && lane == 0) {
-        float* p = reinterpret_cast<float*>(out & ~(uintptr_t)3);
-        p[0] = rf;
-        if (out & 1) p[-1] = rf;
-        if (out & 2) p[1] = rf;
+    return rf;
+}
+
+#if NB_ARITH_FAST
+// sample_n (nebula3d.py:195-226) on a grid of fewer than 2^31 cells, for positions in the domain, with
+// the position already in cells: (gx, gy, gz) = p / dx - 1/2.  The lower corner is clamped to n - 2, so
+// the eight corners lie at fixed steps from one address and none needs a clamp of its own; the
+// fractions saturate to [0, 1], which gives the edge cell's value beyond the outermost centres as
+// clamped corners do.  floor(g) is g - 1/2 rounded to an integer by adding 1.5 x 2^23 (at a cell centre
+// either cell may be the lower corner: a fraction of 0 or 1), whose bits also hold the index: no
+// conversion instruction (those issue at an eighth of the rate).
+struct CellSampler {
+    const float* base;
+    float hx, hy, hz;           // the largest lower corner along each axis
+    int ny, nz, sy, sx;         // steps to the upper corner along j and i (0 on a one-cell axis)
+    unsigned k;                 // the rounding constant's share of an index
+    __device__ __forceinline__ CellSampler(const NbConst& C, const float* rho) {
+        const unsigned M = 0x4B400000u;                      // the bits of 1.5 x 2^23
+        base = rho;
+        hx = (float)max(C.nx - 2, 0);
+        hy = (float)max(C.ny - 2, 0);
+        hz = (float)(C.nz - 2);
+        ny = C.ny;
+        nz = C.nz;
+        sy = C.ny > 1 ? C.nz : 0;
+        sx = C.nx > 1 ? C.ny * C.nz : 0;
+        k = (M * (unsigned)ny + M) * (unsigned)nz + M;
+    }
+    __device__ __forceinline__ float operator()(float gx, float gy, float gz) const {
+        const float M = 12582912.0f;
+        const float mx = fminf(fmaxf(gx - 0.5f, -0.5f), hx) + M, my = fminf(fmaxf(gy - 0.5f, -0.5f), hy) + M;
+        const float mz = fminf(fmaxf(gz - 0.5f, -0.5f), hz) + M;
+        const float fx = __saturatef(gx - (mx - M)), fy = __saturatef(gy - (my - M)), fz = __saturatef(gz - (mz - M));
+        const unsigned e = (__float_as_uint(mx) * (unsigned)ny + __float_as_uint(my)) * (unsigned)nz +
+                           __float_as_uint(mz) - k;
+        const float *p00 = base + e, *p01 = p00 + sy, *p10 = p00 + sx, *p11 = p10 + sy;
+        const F2 a0 = mk2(__ldg(p00), __ldg(p00 + 1)), a1 = mk2(__ldg(p10), __ldg(p10 + 1));
+        const F2 b0 = mk2(__ldg(p01), __ldg(p01 + 1)), b1 = mk2(__ldg(p11), __ldg(p11 + 1));
+        const F2 x2 = mk2(fx, fx), y2 = mk2(fy, fy);
+        const F2 a = vfma(vsub(a1, a0), x2, a0), b = vfma(vsub(b1, b0), x2, b0), c = vfma(vsub(b, a), y2, a);
+        return fmaf(hi(c) - lo(c), fz, lo(c));
+    }
+};
+
+// nebula3d.py:247-270 cast_rays, one lane per ray, on a grid of fewer than 2^31 cells: the march takes
+// only the samples inside the box (outside it the density is 0: they add nothing), so no sample is
+// tested against the domain.
+__device__ __forceinline__ float cast_ray1(const NbConst& C, const float4 d, const float* __restrict__ rho, float sx,
+                                           float sy, float sz, float Q) {
+    const float dr = C.dr_f;
+    float t0 = 0.0f, t1 = 1e9f;
+    const float o[3] = {sx, sy, sz}, dd[3] = {d.x, d.y, d.z};
+    // the box as sample_n's float32 test of p / dx - 1/2 sees it: a position rounds onto a face from half an
+    // ulp outside it (which decides for rays that run in a face)
+    const float e0 = -C.dx * 0x1p-25f, e1 = 1.0f + 0x1p-23f;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {                        // nebula3d.py:229-244 box_range
+        if (fabsf(dd[a]) < 1e-9f) {
+            if (o[a] < 0.0f || o[a] > C.bmax[a]) t1 = -1.0f;
+        } else {
+            const float inv = rcp_approx(dd[a]), ta = (e0 - o[a]) * inv, tb = (C.bmax[a] * e1 - o[a]) * inv;
+            t0 = fmaxf(t0, fminf(ta, tb));
+            t1 = fminf(t1, fmaxf(ta, tb));
+        }
+    }
+    // samples lie at (n + 1/2) dr; n is kept as the float n + 1/2 (exact below 2^23)
+    const float inv_dr = rcp_approx(dr);
+    float nf = fmaxf(ceilf(t0 * inv_dr - 0.5f), 0.0f) + 0.5f;
+    const float n1 = fminf(t1 * inv_dr, (float)C.nsteps - 0.5f);
+    const CellSampler at(C, rho);
+    const float inv_dx = C.dx_pow2 ? C.inv_dx : rcp_approx(C.dx);
+    float sum = 0.0f, comp = 0.0f, rf = C.diag_f;        // Kahan-compensated column
+    for (; nf <= n1; nf += 1.0f) {
+        const float r = nf * dr;
+        // the position first, then in cells, and the product in the reference's order: the fronts are those
+        // of the general form to the bit but where a sample lies on a cell centre or in the outermost half
+        // cell.  (Folding both into one multiply-add moves fronts by 3e-7 of the box, which a stiff front
+        // amplifies to 1e-3 of the momentum in single cells within a few steps.)
+        const float nv = at(fmaf(fmaf(d.x, r, sx), inv_dx, -0.5f), fmaf(fmaf(d.y, r, sy), inv_dx, -0.5f),
+                            fmaf(fmaf(d.z, r, sz), inv_dx, -0.5f));
+        const float inc = nv * nv * r * r * dr, col = sum - comp;
+        if (col + inc > Q) {
+            rf = r - 0.5f * dr + dr * (Q - col) / fmaxf(inc, 1e-20f);
+            break;
+        }
+        const float y = inc - comp, t = sum + y;
+        comp = (t - sum) - y;
+        sum = t;
+    }
+    return rf;
+}
+#endif
+
+// The direction (iu, ip) of a star's q-th ray.  A warp takes 8 (u) x 4 (phi) neighbouring directions
+// where the ray grid divides so: the bundle stays within a few cells, so its rays share cache lines and
+// end within a few samples of one another, and its fronts fill whole sectors of the [phi][u] table (32
+// neighbours along phi span an arc ten times as wide).  With CellSampler (225 instead of 380 thread
+// instructions a cell at 192^3): cast_rays 118 -> 78 us at 256^3, 105 -> 69 at 192^3, 59 -> 48 at 64^3;
+// the exact build, whose sampler stays, is level.
+__device__ __forceinline__ int2 ray_dir(int q, int nu, int nphi) {
+    if ((nu & 7) || (nphi & 3)) {
+        const int iu = q / nphi;
+        return make_int2(iu, q - iu * nphi);
+    }
+    const int t = q >> 5, l = q & 31, tu = nu >> 3, tp = t / tu;
+    return make_int2((t - tp * tu) * 8 + (l & 7), tp * 4 + (l >> 3));
+}
+
+// Each star's least and largest front radius, for apply_front's culling: order-preserving bits of the
+// floats (a NaN orders above every number), merged by one minimum and one maximum per warp.
+__device__ __forceinline__ unsigned front_key(float v) {
+    const unsigned b = __float_as_uint(v);
+    return b ^ ((b >> 31) ? 0xffffffffu : 0x80000000u);
+}
+__device__ __forceinline__ float front_of_key(unsigned k) {
+    return __uint_as_float(k ^ ((k >> 31) ? 0x80000000u : 0xffffffffu));
+}
+// Every thread of the block calls it; `on`: the lane holds a front of star s of `bounds`, `id` tells the
+// stars of a block apart.  A block whose rays are all one star's merges once: two atomics per warp on a
+// handful of addresses took longer than the marches (133 us at every grid size).
+__device__ __forceinline__ void merge_front(uint2* bounds, int id, int s, float rf, bool on) {
+    __shared__ unsigned part[2][8];
+    __shared__ int first;
+    if (threadIdx.x == 0) first = id;
+    __syncthreads();
+    const unsigned k = front_key(rf);
+    if (__syncthreads_and(on && id == first)) {
+        const unsigned mn = __reduce_min_sync(0xffffffffu, k), mx = __reduce_max_sync(0xffffffffu, k);
+        if ((threadIdx.x & 31) == 0) {
+            part[0][threadIdx.x >> 5] = mn;
+            part[1][threadIdx.x >> 5] = mx;
+        }
+        __syncthreads();
+        if (threadIdx.x < 8) {
+            const unsigned m = __reduce_min_sync(0xffu, part[0][threadIdx.x]);
+            const unsigned x = __reduce_max_sync(0xffu, part[1][threadIdx.x]);
+            if (threadIdx.x == 0) {
+                atomicMin(&bounds[s].x, m);
+                atomicMax(&bounds[s].y, x);
+            }
+        }
+    } else if (on) {
+        atomicMin(&bounds[s].x, k);
+        atomicMax(&bounds[s].y, k);
     }
 }
 
-// Where the front of ray (iu, ip) of star s goes in an instance's table [star][phi][u]: one float,
-// or (pairs) the .x of its own float2 pair, flagged to write the .y of the pair below it too (and
-// of its own at the last u).
-__device__ __forceinline__ uintptr_t front_slot(float* rfront, bool pairs, int s, long long nray, int nu, int iu,
-                                                int ip) {
+// The front of ray (iu, ip) of star s into an instance's table [star][phi][u]: one float, or (pairs)
+// the .x of its own float2 pair and the .y of the pair below it (and of its own at the last u).
+__device__ __forceinline__ void put_front(float* rfront, bool pairs, int s, long long nray, int nu, int iu, int ip,
+                                          float rf) {
     const long long e = (long long)s * nray + (long long)ip * nu + iu;
-    if (!pairs) return reinterpret_cast<uintptr_t>(rfront + e);
-    return reinterpret_cast<uintptr_t>(rfront + 2 * e) | (iu > 0 ? 1u : 0u) | (iu == nu - 1 ? 2u : 0u);
+    if (!pairs) {
+        rfront[e] = rf;
+        return;
+    }
+    float* p = rfront + 2 * e;
+    p[0] = rf;
+    if (iu > 0) p[-1] = rf;
+    if (iu == nu - 1) p[1] = rf;
+}
+
+// The front radius of direction (iu, ip) of a star.  SMALL: the one-lane form of the fast build.
+template <int G, bool SMALL>
+__device__ __forceinline__ float cast_dir(const NbConst& C, const float4* __restrict__ dirs,
+                                          const float* __restrict__ rho, int2 dir, float sx, float sy, float sz, float Q,
+                                          int lane, unsigned gmask, bool live) {
+    const int ray = dir.x * C.nphi + dir.y;
+#if NB_ARITH_FAST
+    if (SMALL) return live ? cast_ray1(C, dirs[ray], rho, sx, sy, sz, Q) : 0.0f;
+#endif
+    return cast_ray<G>(C, dirs, rho, ray, sx, sy, sz, Q, lane, gmask, live);
 }
 
 // Resident blocks per SM of the ray kernel: 5 (48 registers); at 6 (40 registers) the warp-uniform
 // march spills 44-84 bytes.
 #define NB_CAST_RAYS_MINB 5
-template <int G, bool PAIRS>
-__global__ void __launch_bounds__(256, NB_CAST_RAYS_MINB) cast_rays_kernel(const NbConst* __restrict__ c, const NbStarW* __restrict__ sw,
-                                                        const float4* __restrict__ dirs,
-                                                        const float* __restrict__ rho, float* __restrict__ rfront,
-                                                        int nstars, const float* star_override, float q_override) {
+template <int G, bool PAIRS, bool SMALL>
+__global__ void __launch_bounds__(256, NB_CAST_RAYS_MINB)
+    cast_rays_kernel(const NbConst* __restrict__ c, const NbStarW* __restrict__ sw, const float4* __restrict__ dirs,
+                     const float* __restrict__ rho, float* __restrict__ rfront, int nstars, uint2* bounds,
+                     const float* star_override, float q_override) {
     const int nray = c->nu * c->nphi;
     const long long gid = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / G;
     const int lane = threadIdx.x % G;
     const unsigned gmask = G == 32 ? 0xffffffffu : (((1u << G) - 1u) << ((threadIdx.x & 31) / G * G));
-    // no early exit: every lane of a warp reaches cast_ray's warp-uniform loop
+    // no early exit: every thread reaches the march's warp-wide operations and the merge's barriers
     const bool in = gid < (long long)nray * nstars;
     // a group index of one instance stays below 2^32 (nb_create checks it): 32-bit division
     const unsigned g32 = in ? (unsigned)gid : 0u;
-    const int s = (int)(g32 / (unsigned)nray), ray = (int)(g32 - (unsigned)s * (unsigned)nray);
+    const int s = (int)(g32 / (unsigned)nray);
+    const int2 dir = ray_dir((int)(g32 - (unsigned)s * (unsigned)nray), c->nu, c->nphi);
     if (star_override) {
-        cast_ray<G>(*c, dirs, rho, reinterpret_cast<uintptr_t>(rfront + ray), ray, star_override[0], star_override[1],
-                    star_override[2], q_override, lane, gmask, in);
+        const float rf = cast_dir<G, SMALL>(*c, dirs, rho, dir, star_override[0], star_override[1], star_override[2],
+                                            q_override, lane, gmask, in);
+        if (in && lane == 0) rfront[dir.x * c->nphi + dir.y] = rf;
         return;
     }
     const NbStarW w = sw[s];
+    const bool live = in && w.active;
+    const float rf = cast_dir<G, SMALL>(*c, dirs, rho, dir, w.w.x, w.w.y, w.w.z, w.q_f, lane, gmask, live);
     // the instance's table is [star][phi][u] (u fastest: the cells of a warp share phi)
-    const int iu = ray / c->nphi, ip = ray - iu * c->nphi;
-    cast_ray<G>(*c, dirs, rho, front_slot(rfront, PAIRS, s, nray, c->nu, iu, ip), ray, w.w.x, w.w.y, w.w.z, w.q_f,
-                lane, gmask, in && w.active);
+    if (live && lane == 0) put_front(rfront, PAIRS, s, nray, c->nu, dir.x, dir.y, rf);
+    if (bounds) merge_front(bounds, s, s, rf, live);
 }
 
 // Rays of every star of every listed instance: job e owns groups [job[e].ray0, job[e+1].ray0).
 // `J` holds the job records (global memory, or the kernel parameter of the param form); the active
 // flags always come from `Jd`, the device copy (they change between replays of a captured step).
-template <int G, typename Jobs>
+template <int G, bool SMALL, typename Jobs>
 __device__ __forceinline__ void cast_rays_batch_body(const Jobs& J, const NbRayJob* __restrict__ Jd, int n_jobs,
                                                      long long n_groups) {
     const long long gid0 = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / G;
     const int lane = threadIdx.x % G;
     const unsigned gmask = G == 32 ? 0xffffffffu : (((1u << G) - 1u) << ((threadIdx.x & 31) / G * G));
-    // no early exit: every lane of a warp reaches cast_ray's warp-uniform loop
+    // no early exit: every thread reaches the march's warp-wide operations and the merge's barriers
     const bool in = gid0 < n_groups;
     const long long gid = in ? gid0 : 0;
     int lo = 0, hi = n_jobs - 1;
@@ -196,27 +358,30 @@ __device__ __forceinline__ void cast_rays_batch_body(const Jobs& J, const NbRayJ
     const int nray = C.nu * C.nphi;
     const long long local = gid - job.ray0;
     const unsigned l32 = (unsigned)local;        // below 2^32 within a job (nb_create): 32-bit division
-    const int s = (int)(l32 / (unsigned)nray), ray = (int)(l32 - (unsigned)s * (unsigned)nray);
+    const int s = (int)(l32 / (unsigned)nray);
+    const int2 dir = ray_dir((int)(l32 - (unsigned)s * (unsigned)nray), C.nu, C.nphi);
     const bool star = in && s < job.nstars && Jd[lo].active;
     NbStarW w{};
     if (star) w = job.sw[s];
-    const int iu = ray / C.nphi, ip = ray - iu * C.nphi;
-    cast_ray<G>(C, job.dirs, job.rho, front_slot(job.rfront, job.pairs != 0, s, nray, C.nu, iu, ip), ray, w.w.x,
-                w.w.y, w.w.z, w.q_f, lane, gmask, star && w.active);
+    const bool live = star && w.active;
+    const float rf = cast_dir<G, SMALL>(C, job.dirs, job.rho, dir, w.w.x, w.w.y, w.w.z, w.q_f, lane, gmask, live);
+    if (live && lane == 0) put_front(job.rfront, job.pairs != 0, s, nray, C.nu, dir.x, dir.y, rf);
+    // the lanes of a warp may belong to two jobs: (job, star) pairs are told apart
+    merge_front(job.front_bounds, lo * NB_MAX_STARS + s, s, rf, live && job.front_bounds);
 }
 
-template <int G>
+template <int G, bool SMALL>
 __global__ void __launch_bounds__(256) cast_rays_batch_kernel(const NbRayJob* __restrict__ jobs, int n_jobs,
                                                               long long n_groups) {
-    cast_rays_batch_body<G>(jobs, jobs, n_jobs, n_groups);
+    cast_rays_batch_body<G, SMALL>(jobs, jobs, n_jobs, n_groups);
 }
 
 // the job records in the kernel parameter (constant bank): 48 registers, 5 blocks / SM
-template <int G>
+template <int G, bool SMALL>
 __global__ void __launch_bounds__(256, NB_CAST_RAYS_MINB)
     cast_rays_batch_param_kernel(const __grid_constant__ NbRayJobs P, const NbRayJob* __restrict__ jobs, int n_jobs,
                                  long long n_groups) {
-    cast_rays_batch_body<G>(P.J, jobs, n_jobs, n_groups);
+    cast_rays_batch_body<G, SMALL>(P.J, jobs, n_jobs, n_groups);
 }
 
 // The stars that can change xi or the front distance of the 32-cell segment [kb, kb + 32) of a
@@ -397,69 +562,10 @@ __device__ __forceinline__ void apply_front_row(const NbConst& C, const float4* 
     }
 }
 
-// Each active star's least and largest front radius over its rays, as NB_FRONT_PARTS partial
-// (least, largest) pairs per star: block (b, s) reduces the b-th slice of star s.  The largest is
-// NaN when a NaN radius was seen (the least skips NaNs).
-// With pair tables a star's slice holds every front twice (as a .x and as a .y): the same set of
-// values, so the same bounds.
-__device__ __forceinline__ void front_bounds_block(const NbStarW* __restrict__ sw, const float* __restrict__ rfront,
-                                                   long long nray, float2* __restrict__ parts, int s, int b) {
-    if (!sw[s].active) return;                  // uniform over the block
-    const float* r = rfront + (long long)s * nray;
-    const long long per = (nray + NB_FRONT_PARTS - 1) / NB_FRONT_PARTS;
-    const long long lo = (long long)b * per, hi = min(nray, lo + per);
-    float mn = __int_as_float(0x7f800000), mx = -mn;
-    bool nan = false;
-    for (long long q = lo + threadIdx.x; q < hi; q += blockDim.x) {
-        const float v = __ldg(r + q);
-        nan |= isnan(v);
-        mn = fminf(mn, v);
-        mx = fmaxf(mx, v);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    }
-    __shared__ float2 wpart[8];
-    const bool any_nan = __syncthreads_or(nan);
-    if ((threadIdx.x & 31) == 0) wpart[threadIdx.x >> 5] = make_float2(mn, mx);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) {
-            mn = fminf(mn, wpart[w].x);
-            mx = fmaxf(mx, wpart[w].y);
-        }
-        parts[s * NB_FRONT_PARTS + b] = make_float2(mn, any_nan ? __int_as_float(0x7fc00000) : mx);
-    }
-}
-
-__global__ void __launch_bounds__(256) front_bounds_kernel(const NbStarW* __restrict__ sw,
-                                                           const float* __restrict__ rfront, long long nray,
-                                                           float2* __restrict__ parts) {
-    front_bounds_block(sw, rfront, nray, parts, blockIdx.y, blockIdx.x);
-}
-
-// the same for every listed instance that culls: block (b, job, star)
-__global__ void __launch_bounds__(256) front_bounds_batch_kernel(const NbRayJob* __restrict__ jobs) {
-    const NbRayJob& J = jobs[blockIdx.y];
-    if (!J.front_parts || !J.active || (int)blockIdx.z >= J.nstars) return;      // uniform over the block
-    front_bounds_block(J.sw, J.rfront, J.pairs ? 2 * J.nray : J.nray, J.front_parts, blockIdx.z, blockIdx.x);
-}
-
-// the partials into (least, largest) per star in shared memory (after load_stars' barrier)
-__device__ __forceinline__ void load_front_bounds(const float2* parts, int nstars, float2* bnd, int tlin) {
-    for (int s = tlin; s < nstars; s += blockDim.x * blockDim.y) {
-        float mn = __int_as_float(0x7f800000), mx = -mn;
-        bool nan = false;
-        for (int b = 0; b < NB_FRONT_PARTS; ++b) {
-            const float2 p = parts[s * NB_FRONT_PARTS + b];
-            mn = fminf(mn, p.x);
-            nan |= isnan(p.y);
-            mx = fmaxf(mx, p.y);
-        }
-        bnd[s] = make_float2(mn, nan ? __int_as_float(0x7fc00000) : mx);
-    }
+// the (least, largest) front radius per star into shared memory (after load_stars' barrier)
+__device__ __forceinline__ void load_front_bounds(const uint2* bounds, int nstars, float2* bnd, int tlin) {
+    for (int s = tlin; s < nstars; s += blockDim.x * blockDim.y)
+        bnd[s] = make_float2(front_of_key(bounds[s].x), front_of_key(bounds[s].y));
     __syncthreads();
 }
 
@@ -478,16 +584,16 @@ __global__ void __launch_bounds__(256, 4) apply_front_kernel(const NbConst* __re
                                                           const NbStarW* __restrict__ sw,
                                                           const float* __restrict__ rfront, int nstars,
                                                           float* __restrict__ xi_raw, void* __restrict__ dfront,
-                                                          unsigned* smax_reset, const float2* __restrict__ parts) {
+                                                          unsigned* smax_reset, const uint2* __restrict__ bounds) {
     __shared__ float4 st[NB_MAX_STARS];
     __shared__ int act[NB_MAX_STARS];
     __shared__ float4 tab[8][NB_ROW_STARS];
     __shared__ float2 bnd[NB_ROW_STARS];
     const int tlin = load_stars(sw, nstars, st, act);
     if (smax_reset && blockIdx.x == 0 && tlin == 0) *smax_reset = 0u;
-    if (parts) load_front_bounds(parts, nstars, bnd, tlin);      // parts only with nstars <= NB_ROW_STARS
+    if (bounds) load_front_bounds(bounds, nstars, bnd, tlin);    // only with nstars <= NB_ROW_STARS
     apply_front_row<PAIRS>(*c, st, act, nstars, rfront, xi_raw, dfront, HALF, blockIdx.x * blockDim.y + threadIdx.y,
-                           tab[threadIdx.y], parts ? bnd : nullptr);
+                           tab[threadIdx.y], bounds ? bnd : nullptr);
 }
 
 // Rows of every listed instance; job e owns blocks [job[e].blk0, job[e+1].blk0) (8 rows each).
@@ -506,13 +612,13 @@ __global__ void __launch_bounds__(256) apply_front_batch_kernel(const NbRayJob* 
     const int lb = (int)(blockIdx.x - J.blk0);
     const int tlin = load_stars(J.sw, J.nstars, st, act);
     if (lb == 0 && tlin == 0) *J.smax = 0u;
-    if (J.front_parts) load_front_bounds(J.front_parts, J.nstars, bnd, tlin);     // uniform over the block
+    if (J.front_bounds) load_front_bounds(J.front_bounds, J.nstars, bnd, tlin);     // uniform over the block
     if (J.pairs)
         apply_front_row<true>(*J.c, st, act, J.nstars, J.rfront, J.xi_raw, J.dfront, J.half != 0,
-                              lb * blockDim.y + threadIdx.y, tab[threadIdx.y], J.front_parts ? bnd : nullptr);
+                              lb * blockDim.y + threadIdx.y, tab[threadIdx.y], J.front_bounds ? bnd : nullptr);
     else
         apply_front_row<false>(*J.c, st, act, J.nstars, J.rfront, J.xi_raw, J.dfront, J.half != 0,
-                               lb * blockDim.y + threadIdx.y, tab[threadIdx.y], J.front_parts ? bnd : nullptr);
+                               lb * blockDim.y + threadIdx.y, tab[threadIdx.y], J.front_bounds ? bnd : nullptr);
 }
 
 // nebula3d.py:310-315 smooth_xi (+ sim.py:941 copy back) of one row, then the CFL max speed
@@ -625,22 +731,25 @@ cudaError_t nb_launch_ray_dirs(int nu, int nphi, float4* dirs, cudaStream_t s) {
 }
 
 cudaError_t nb_launch_cast_rays(const NbConst* c, const NbStarW* sw, const float4* dirs, const float* rho,
-                                float* rfront, int nstars, int group, const float* star_override, float q_override,
-                                cudaStream_t s, int nu, int nphi, int pairs) {
+                                float* rfront, int nstars, int group, uint2* bounds, const float* star_override,
+                                float q_override, cudaStream_t s, int nu, int nphi, int pairs, int small) {
     const long long threads = (long long)nu * nphi * nstars * group;
     const int blocks = (int)((threads + 255) / 256);
-#define NB_RAYS_LAUNCH(G)                                                                                      \
-    (pairs ? cast_rays_kernel<G, true><<<blocks, 256, 0, s>>>(c, sw, dirs, rho, rfront, nstars, star_override,  \
-                                                              q_override)                                       \
-           : cast_rays_kernel<G, false><<<blocks, 256, 0, s>>>(c, sw, dirs, rho, rfront, nstars, star_override, \
-                                                               q_override))
+#define NB_RAYS_LAUNCH(G, SM)                                                                                      \
+    (pairs ? cast_rays_kernel<G, true, SM><<<blocks, 256, 0, s>>>(c, sw, dirs, rho, rfront, nstars, bounds,         \
+                                                                  star_override, q_override)                        \
+           : cast_rays_kernel<G, false, SM><<<blocks, 256, 0, s>>>(c, sw, dirs, rho, rfront, nstars, bounds,        \
+                                                                   star_override, q_override))
     switch (group) {
-        case 1: NB_RAYS_LAUNCH(1); break;
-        case 2: NB_RAYS_LAUNCH(2); break;
-        case 4: NB_RAYS_LAUNCH(4); break;
-        case 8: NB_RAYS_LAUNCH(8); break;
-        case 16: NB_RAYS_LAUNCH(16); break;
-        default: NB_RAYS_LAUNCH(32); break;
+        case 1:
+            if (NB_RAYS_SMALL && small) NB_RAYS_LAUNCH(1, NB_RAYS_SMALL);
+            else NB_RAYS_LAUNCH(1, false);
+            break;
+        case 2: NB_RAYS_LAUNCH(2, false); break;
+        case 4: NB_RAYS_LAUNCH(4, false); break;
+        case 8: NB_RAYS_LAUNCH(8, false); break;
+        case 16: NB_RAYS_LAUNCH(16, false); break;
+        default: NB_RAYS_LAUNCH(32, false); break;
     }
 #undef NB_RAYS_LAUNCH
     return cudaGetLastError();
@@ -648,23 +757,18 @@ cudaError_t nb_launch_cast_rays(const NbConst* c, const NbStarW* sw, const float
 
 cudaError_t nb_launch_apply_front(const NbConst* c, const NbStarW* sw, const float* rfront, int nstars,
                                   float* xi_raw, void* dfront, unsigned* smax_reset, cudaStream_t s, int nx, int ny,
-                                  int half, float2* front_parts, long long nray, int pairs) {
+                                  int half, const uint2* bounds, int pairs) {
     const dim3 blk(32, 8);
     const int blocks = rowwalk_blocks(nx, ny);
-    const float2* parts = nullptr;
-    if (front_parts && nstars >= 1 && nstars <= NB_ROW_STARS) {
-        front_bounds_kernel<<<dim3(NB_FRONT_PARTS, nstars), 256, 0, s>>>(sw, rfront, pairs ? 2 * nray : nray,
-                                                                          front_parts);
-        parts = front_parts;
-    }
+    if (nstars < 1 || nstars > NB_ROW_STARS) bounds = nullptr;
     if (half && pairs)
-        apply_front_kernel<true, true><<<blocks, blk, 0, s>>>(c, sw, rfront, nstars, xi_raw, dfront, smax_reset, parts);
+        apply_front_kernel<true, true><<<blocks, blk, 0, s>>>(c, sw, rfront, nstars, xi_raw, dfront, smax_reset, bounds);
     else if (half)
-        apply_front_kernel<true, false><<<blocks, blk, 0, s>>>(c, sw, rfront, nstars, xi_raw, dfront, smax_reset, parts);
+        apply_front_kernel<true, false><<<blocks, blk, 0, s>>>(c, sw, rfront, nstars, xi_raw, dfront, smax_reset, bounds);
     else if (pairs)
-        apply_front_kernel<false, true><<<blocks, blk, 0, s>>>(c, sw, rfront, nstars, xi_raw, dfront, smax_reset, parts);
+        apply_front_kernel<false, true><<<blocks, blk, 0, s>>>(c, sw, rfront, nstars, xi_raw, dfront, smax_reset, bounds);
     else
-        apply_front_kernel<false, false><<<blocks, blk, 0, s>>>(c, sw, rfront, nstars, xi_raw, dfront, smax_reset, parts);
+        apply_front_kernel<false, false><<<blocks, blk, 0, s>>>(c, sw, rfront, nstars, xi_raw, dfront, smax_reset, bounds);
     return cudaGetLastError();
 }
 
@@ -675,7 +779,7 @@ cudaError_t nb_launch_smooth(const NbConst* c, const float* xi_raw, float* xi, c
 }
 
 cudaError_t nb_launch_ionize_batch(const NbRayJob* jobs, const NbRayJob* host_jobs, int n_jobs, long long n_groups,
-                                   long long n_blocks, int group, cudaStream_t s) {
+                                   long long n_blocks, int group, int small, cudaStream_t s) {
     if (n_jobs <= 0) return cudaSuccess;
     const long long threads = n_groups * group;
     const long long blocks = (threads + 255) / 256;
@@ -685,24 +789,33 @@ cudaError_t nb_launch_ionize_batch(const NbRayJob* jobs, const NbRayJob* host_jo
         std::memcpy(P.J, host_jobs, sizeof(NbRayJob) * n_jobs);
         const unsigned nb = (unsigned)blocks;
         switch (group) {
-            case 1: cast_rays_batch_param_kernel<1><<<nb, 256, 0, s>>>(P, jobs, n_jobs, n_groups); break;
-            case 2: cast_rays_batch_param_kernel<2><<<nb, 256, 0, s>>>(P, jobs, n_jobs, n_groups); break;
-            case 4: cast_rays_batch_param_kernel<4><<<nb, 256, 0, s>>>(P, jobs, n_jobs, n_groups); break;
-            case 8: cast_rays_batch_param_kernel<8><<<nb, 256, 0, s>>>(P, jobs, n_jobs, n_groups); break;
-            case 16: cast_rays_batch_param_kernel<16><<<nb, 256, 0, s>>>(P, jobs, n_jobs, n_groups); break;
-            default: cast_rays_batch_param_kernel<32><<<nb, 256, 0, s>>>(P, jobs, n_jobs, n_groups); break;
+            case 1:
+                if (NB_RAYS_SMALL && small)
+                    cast_rays_batch_param_kernel<1, NB_RAYS_SMALL><<<nb, 256, 0, s>>>(P, jobs, n_jobs, n_groups);
+                else
+                    cast_rays_batch_param_kernel<1, false><<<nb, 256, 0, s>>>(P, jobs, n_jobs, n_groups);
+                break;
+            case 2: cast_rays_batch_param_kernel<2, false><<<nb, 256, 0, s>>>(P, jobs, n_jobs, n_groups); break;
+            case 4: cast_rays_batch_param_kernel<4, false><<<nb, 256, 0, s>>>(P, jobs, n_jobs, n_groups); break;
+            case 8: cast_rays_batch_param_kernel<8, false><<<nb, 256, 0, s>>>(P, jobs, n_jobs, n_groups); break;
+            case 16: cast_rays_batch_param_kernel<16, false><<<nb, 256, 0, s>>>(P, jobs, n_jobs, n_groups); break;
+            default: cast_rays_batch_param_kernel<32, false><<<nb, 256, 0, s>>>(P, jobs, n_jobs, n_groups); break;
         }
     } else if (blocks > 0) {
         switch (group) {
-            case 1: cast_rays_batch_kernel<1><<<(unsigned)blocks, 256, 0, s>>>(jobs, n_jobs, n_groups); break;
-            case 2: cast_rays_batch_kernel<2><<<(unsigned)blocks, 256, 0, s>>>(jobs, n_jobs, n_groups); break;
-            case 4: cast_rays_batch_kernel<4><<<(unsigned)blocks, 256, 0, s>>>(jobs, n_jobs, n_groups); break;
-            case 8: cast_rays_batch_kernel<8><<<(unsigned)blocks, 256, 0, s>>>(jobs, n_jobs, n_groups); break;
-            case 16: cast_rays_batch_kernel<16><<<(unsigned)blocks, 256, 0, s>>>(jobs, n_jobs, n_groups); break;
-            default: cast_rays_batch_kernel<32><<<(unsigned)blocks, 256, 0, s>>>(jobs, n_jobs, n_groups); break;
+            case 1:
+                if (NB_RAYS_SMALL && small)
+                    cast_rays_batch_kernel<1, NB_RAYS_SMALL><<<(unsigned)blocks, 256, 0, s>>>(jobs, n_jobs, n_groups);
+                else
+                    cast_rays_batch_kernel<1, false><<<(unsigned)blocks, 256, 0, s>>>(jobs, n_jobs, n_groups);
+                break;
+            case 2: cast_rays_batch_kernel<2, false><<<(unsigned)blocks, 256, 0, s>>>(jobs, n_jobs, n_groups); break;
+            case 4: cast_rays_batch_kernel<4, false><<<(unsigned)blocks, 256, 0, s>>>(jobs, n_jobs, n_groups); break;
+            case 8: cast_rays_batch_kernel<8, false><<<(unsigned)blocks, 256, 0, s>>>(jobs, n_jobs, n_groups); break;
+            case 16: cast_rays_batch_kernel<16, false><<<(unsigned)blocks, 256, 0, s>>>(jobs, n_jobs, n_groups); break;
+            default: cast_rays_batch_kernel<32, false><<<(unsigned)blocks, 256, 0, s>>>(jobs, n_jobs, n_groups); break;
         }
     }
-    front_bounds_batch_kernel<<<dim3(NB_FRONT_PARTS, n_jobs, NB_ROW_STARS), 256, 0, s>>>(jobs);
     apply_front_batch_kernel<<<(unsigned)n_blocks, dim3(32, 8), 0, s>>>(jobs, n_jobs);
     smooth_batch_kernel<<<(unsigned)n_blocks, dim3(32, 8), 0, s>>>(jobs, n_jobs);
     return cudaGetLastError();

@@ -42,9 +42,10 @@ __device__ void star_weight(const NbConst& c, const NbStarDev& s, double t, NbSt
 // NB_ADV_PRE = a stirring-phase step (sim.py:1044-1050: dt without dt_cap, tp += dt)
 __device__ __forceinline__ void ctrl_body(const NbConst* __restrict__ c, NbState* __restrict__ st,
                                           const NbStarDev* __restrict__ stars, NbStarW* __restrict__ sw, int nstars,
-                                          int advance) {
+                                          int advance, uint2* bounds) {
     const double t = st->t;
     for (int s = threadIdx.x; s < nstars; s += blockDim.x) star_weight(*c, stars[s], t, sw[s]);
+    if (bounds && !advance && threadIdx.x < NB_ROW_STARS) bounds[threadIdx.x] = make_uint2(0xffffffffu, 0u);
     __syncthreads();                                      // every thread has read t before it moves
     if (!advance || threadIdx.x != 0) return;
     const bool pre = advance == NB_ADV_PRE;
@@ -102,8 +103,8 @@ __device__ __forceinline__ void ctrl_body(const NbConst* __restrict__ c, NbState
 
 __global__ void ctrl_kernel(const NbConst* __restrict__ c, NbState* __restrict__ st,
                             const NbStarDev* __restrict__ stars, NbStarW* __restrict__ sw, int nstars,
-                            int advance) {
-    ctrl_body(c, st, stars, sw, nstars, advance);
+                            int advance, uint2* bounds) {
+    ctrl_body(c, st, stars, sw, nstars, advance, bounds);
 }
 
 // one block per instance of a batch; block 0 also resets the persistent stage kernels' counters
@@ -114,7 +115,7 @@ __global__ void ctrl_batch_kernel(const NbBatchInst* __restrict__ insts, int n, 
         counters[1] = 0u;
     }
     if (!I.active) return;                       // an idle slot: its clock stays
-    ctrl_body(I.c, I.st, I.stars, I.sw, I.nstars, advance);
+    ctrl_body(I.c, I.st, I.stars, I.sw, I.nstars, advance, I.bounds);
 }
 
 // nebula3d.py:154-162 max_speed, as an exact max reduction (atomicMax on the bits of a
@@ -187,13 +188,13 @@ __global__ void reduce_final(const double* __restrict__ part, int nb, double* __
 
 cudaError_t nb_launch_ctrl(const NbConst* c, NbState* st, const NbStarDev* stars, NbStarW* sw, int nstars,
                            int advance, cudaStream_t s) {
-    ctrl_kernel<<<1, 128, 0, s>>>(c, st, stars, sw, nstars, advance);
+    ctrl_kernel<<<1, 128, 0, s>>>(c, st, stars, sw, nstars, advance, nullptr);
     return cudaGetLastError();
 }
 
 cudaError_t nb_launch_weights(const NbConst* c, const NbState* st, const NbStarDev* stars, NbStarW* sw,
-                              int nstars, cudaStream_t s) {
-    ctrl_kernel<<<1, 128, 0, s>>>(c, const_cast<NbState*>(st), stars, sw, nstars, 0);
+                              int nstars, uint2* bounds, cudaStream_t s) {
+    ctrl_kernel<<<1, 128, 0, s>>>(c, const_cast<NbState*>(st), stars, sw, nstars, 0, bounds);
     return cudaGetLastError();
 }
 
