@@ -216,7 +216,7 @@ int do_ionize(nb_instance* h) {
         Prof pf(h, NB_PROF_CAST_RAYS, 1);
         CK(h, nb_launch_cast_rays(h->c, h->sw, h->dirs, f.rho, h->rfront, h->nstars, h->ray_group,
                                   cull ? h->front_bounds : nullptr, nullptr, 0.0f, h->stream, h->d.nu, h->d.nphi,
-                                  h->front_pairs, h->ncell < (1LL << 31)));
+                                  h->front_pairs, nb_rays_small(h->hc)));
     }
     if (h->hc.plane_on) {
         Prof pf(h, NB_PROF_CAST_RAYS, 1);
@@ -404,10 +404,15 @@ NB_EXPORT int nb_create(const nb_desc* d, nb_handle* out) {
             return bail(NB_ERR_CUDA);
         }
     CKC(cudaMemcpyAsync(h->maps, hm, sizeof(hm), cudaMemcpyHostToDevice, h->stream));
-    CKC(nb_launch_ray_dirs(d->nu, d->nphi, h->dirs, h->stream));
     CKC(nb_launch_ray_dirs(d->fnu, d->fnphi, h->dirs_fuv, h->stream));
     CKC(cudaMemcpyAsync(h->c, &h->hc, sizeof(NbConst), cudaMemcpyHostToDevice, h->stream));
-    CKC(cudaStreamSynchronize(h->stream));
+    float4* unordered = nullptr;
+    CKC(cudaMalloc(&unordered, sizeof(float4) * (size_t)d->nu * d->nphi));
+    e = nb_launch_ray_dirs(d->nu, d->nphi, unordered, h->stream);
+    if (e == cudaSuccess) e = nb_launch_ray_order(d->nu, d->nphi, unordered, h->dirs, h->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    cudaFree(unordered);
+    CKC(e);
 #undef CKC
     *out = h;
     return NB_OK;
@@ -807,7 +812,7 @@ NB_EXPORT int nb_cast_rays(nb_handle h, const double xyz[3], double Q, float* rf
     float s3[4] = {(float)xyz[0], (float)xyz[1], (float)xyz[2], 0.f};
     CK(h, cudaMemcpyAsync(h->scratch3, s3, sizeof(s3), cudaMemcpyHostToDevice, h->stream));
     CK(h, nb_launch_cast_rays(h->c, h->sw, h->dirs, h->d.f.rho, rfront_out, 1, h->ray_group, nullptr, h->scratch3,
-                              (float)Q, h->stream, h->d.nu, h->d.nphi, 0, h->ncell < (1LL << 31)));
+                              (float)Q, h->stream, h->d.nu, h->d.nphi, 0, nb_rays_small(h->hc)));
     CK(h, cudaStreamSynchronize(h->stream));
     return NB_OK;
 }
@@ -977,7 +982,7 @@ struct nb_batch_s {
     cudaStream_t bs = nullptr;          // the batch's own stream (capturable)
     cudaEvent_t ev_in = nullptr, ev_out = nullptr;
     int solver = 0, limiter = 0, max_stars = 1, grid = 0, ray_group = 1;
-    int small = 1;                      // every instance below 2^31 cells (the ray cast's 32-bit indices)
+    int small = 1;                      // nb_rays_small of every instance
     int idx32 = 1;                      // 32-bit offsets reach every instance's cells
     NbBatchInst* d_inst = nullptr;
     HydroLaunch* d_L1 = nullptr;
@@ -1176,7 +1181,7 @@ NB_EXPORT int nb_batch_create(const nb_handle* hs, const int* ion_every, int n, 
         b->max_stars = std::max(b->max_stars, h->nstars);
         b->n_plane += h->hc.plane_on ? 1 : 0;
         if (!nb_hydro_idx32(h->ncell)) b->idx32 = 0;
-        if (h->ncell >= (1LL << 31)) b->small = 0;
+        if (!nb_rays_small(h->hc)) b->small = 0;
     }
     const int params = b->idx32 && n <= NB_BATCH_PARAM_MAX;
     b->grid = sm_count() * nb_hydro_batch_blocks_per_sm(b->solver, b->limiter, b->max_stars, b->idx32, params);

@@ -1,5 +1,5 @@
 // Paired FP32 (sm_100+ add/sub/mul/fma.rn.f32x2): one instruction issue for two float operations.
-// Fast build only: alone each rounds as the scalar operation, but the assembler fuses a dependent
+// The pairs are for the fast build only: alone each rounds as the scalar operation, but the assembler fuses a dependent
 // mul.rn.f32x2 -> add.rn.f32x2 into one multiply-add even with -fmad=false.
 #pragma once
 

@@ -274,9 +274,11 @@ cudaError_t nb_launch_render_pack(const NbConst* c, const float* rho, const floa
                                   const nb_pack_params& pp, int shock_on, int smooth, void* out8, void* tmp8, int nx,
                                   int ny, cudaStream_t s);
 cudaError_t nb_launch_ray_dirs(int nu, int nphi, float4* dirs, cudaStream_t s);
+// the directions in the order of the ionizing ray cast, each with its place in the front table
+cudaError_t nb_launch_ray_order(int nu, int nphi, const float4* dirs, float4* out, cudaStream_t s);
 // pairs: the instance's front table holds (rf(u), rf(u + 1)) float2 pairs (2 * nu * nphi floats per
-// star); a star_override launch writes the reference layout [u][phi] (pairs = 0); small: fewer than
-// 2^31 cells
+// star); a star_override launch writes the reference layout [u][phi] (pairs = 0); small: nb_rays_small
+int nb_rays_small(const NbConst& c);
 cudaError_t nb_launch_cast_rays(const NbConst* c, const NbStarW* sw, const float4* dirs, const float* rho,
                                 float* rfront, int nstars, int group, uint2* bounds, const float* star_override,
                                 float q_override, cudaStream_t s, int nu, int nphi, int pairs, int small);

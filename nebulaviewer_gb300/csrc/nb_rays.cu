@@ -9,7 +9,7 @@
 //    carry (G > 1: an inclusive group scan; two lanes take it from one exchange), and the
 //    first sample whose column passes Q is found with one ballot.  That march is warp-uniform: a
 //    warp's groups loop together until all are done, and the trilinear sampler has no branches.
-//    The fast build's one-lane march (cast_ray1) is a plain loop of its own.
+//    The one-lane march (cast_ray1) is a plain loop of its own.
 //    All rays of all active stars are one launch, a warp a bundle of neighbouring directions.
 //  * The front table holds, per (star, phi, u), the pair (rf(u), rf(min(u + 1, nu - 1))) as one
 //    float2 (cast_rays writes each front into its own pair and its lower neighbour's), so the
@@ -24,15 +24,19 @@
 //    (nebula3d.py:154-162), so an ionizing step needs no separate max-speed pass.
 #include <cstring>
 
-#include "nb_rayutil.cuh"
-#if defined(NB_ARITH_FAST) && NB_ARITH_FAST
 #include "nb_f32x2.cuh"
-#define NB_RAYS_SMALL true         // the fast build's one-lane march on grids of fewer than 2^31 cells
-#else
-#define NB_RAYS_SMALL false
-#endif
+#include "nb_rayutil.cuh"
 
 namespace {
+
+// The place of direction (iu, ip) in the order of the ionizing ray cast.  A warp takes 8 (u) x 4 (phi)
+// neighbouring directions where the ray grid divides so: the bundle stays within a few cells, so its rays
+// share cache lines and end within a few samples of one another, and its fronts fill whole sectors of the
+// [phi][u] table (32 neighbours along phi span an arc ten times as wide).
+__device__ __forceinline__ int ray_place(int iu, int ip, int nu, int nphi) {
+    if ((nu & 7) || (nphi & 3)) return iu * nphi + ip;
+    return (((ip >> 2) * (nu >> 3) + (iu >> 3)) << 5) + (ip & 3) * 8 + (iu & 7);
+}
 
 // Ray directions of nebula3d.py:253-256 / 329-332 in float32; cos/sin of the float32 angle
 // are evaluated in FP64 and rounded (the correctly rounded float32 value in all but
@@ -47,20 +51,30 @@ __global__ void ray_dirs_kernel(int nu, int nphi, float4* __restrict__ dirs) {
     const float cph = (float)cos((double)phi), sph = (float)sin((double)phi);
     dirs[id] = make_float4(s * cph, s * sph, u, 0.0f);
 }
+// The directions in the order of the ionizing ray cast (a kernel of its own: with other stores in
+// ray_dirs_kernel the fast build rounds u differently at some nu); .w: the direction's place ip * nu + iu in a
+// [phi][u] table, its sign bit set at the first and last u (the cast does no index division).
+__global__ void ray_order_kernel(int nu, int nphi, const float4* __restrict__ dirs, float4* __restrict__ out) {
+    const int id = blockIdx.x * blockDim.x + threadIdx.x;
+    if (id >= nu * nphi) return;
+    const int iu = id / nphi, ip = id % nphi;
+    const int w = (ip * nu + iu) | (iu == 0 || iu == nu - 1 ? 0x80000000 : 0);
+    float4 d = dirs[id];
+    d.w = __int_as_float(w);
+    out[ray_place(iu, ip, nu, nphi)] = d;
+}
 
-// nebula3d.py:247-270 cast_rays: ray `ray` of star (sx, sy, sz, Q), G lanes per ray; every
+// nebula3d.py:247-270 cast_rays: the ray along d of star (sx, sy, sz, Q), G lanes per ray; every
 // lane of the group gets the front radius.
 template <int G>
-__device__ __forceinline__ float cast_ray(const NbConst& C, const float4* __restrict__ dirs,
-                                         const float* __restrict__ rho, int ray, float sx, float sy,
-                                         float sz, float Q, int lane, unsigned gmask, bool live) {
+__device__ __forceinline__ float cast_ray(const NbConst& C, const float4 d, const float* __restrict__ rho, float sx,
+                                         float sy, float sz, float Q, int lane, unsigned gmask, bool live) {
     // Warp-uniform march: every lane of the warp runs the loop until all of its groups are done
-    // (`live` false: the group has no ray; `ray` is then any valid index), a finished group's lanes
+    // (`live` false: the group has no ray), a finished group's lanes
     // only carry predicated-off values, so the warp never diverges inside the loop.
     const int nx = C.nx, ny = C.ny, nz = C.nz;
     const float dx = C.dx, inv_dx = C.inv_dx, dr = C.dr_f;
     const bool pow2 = C.dx_pow2 != 0;
-    const float4 d = dirs[ray];
     float t0, t1;
     nb_box_range(sx, sy, sz, d.x, d.y, d.z, C.bmax, t0, t1);
     const int n0 = trunc_i(t0 / dr);
@@ -133,109 +147,118 @@ __device__ __forceinline__ float cast_ray(const NbConst& C, const float4* __rest
     return rf;
 }
 
+// c + a b, as the build contracts it
+__device__ __forceinline__ float mac(float a, float b, float c) {
 #if NB_ARITH_FAST
-// sample_n (nebula3d.py:195-226) on a grid of fewer than 2^31 cells, for positions in the domain, with
-// the position already in cells: (gx, gy, gz) = p / dx - 1/2.  The lower corner is clamped to n - 2, so
-// the eight corners lie at fixed steps from one address and none needs a clamp of its own; the
-// fractions saturate to [0, 1], which gives the edge cell's value beyond the outermost centres as
-// clamped corners do.  floor(g) is g - 1/2 rounded to an integer by adding 1.5 x 2^23 (at a cell centre
-// either cell may be the lower corner: a fraction of 0 or 1), whose bits also hold the index: no
-// conversion instruction (those issue at an eighth of the rate).
-struct CellSampler {
-    const float* base;
-    float hx, hy, hz;           // the largest lower corner along each axis
-    int ny, nz, sy, sx;         // steps to the upper corner along j and i (0 on a one-cell axis)
-    unsigned k;                 // the rounding constant's share of an index
-    __device__ __forceinline__ CellSampler(const NbConst& C, const float* rho) {
-        const unsigned M = 0x4B400000u;                      // the bits of 1.5 x 2^23
-        base = rho;
-        hx = (float)max(C.nx - 2, 0);
-        hy = (float)max(C.ny - 2, 0);
-        hz = (float)(C.nz - 2);
-        ny = C.ny;
-        nz = C.nz;
-        sy = C.ny > 1 ? C.nz : 0;
-        sx = C.nx > 1 ? C.ny * C.nz : 0;
-        k = (M * (unsigned)ny + M) * (unsigned)nz + M;
+    return fmaf(a, b, c);
+#else
+    return vadd(c, vmul(a, b));
+#endif
+}
+// sample_n and the sample range out of line: cast_ray1 needs them only near the box's faces
+__device__ __noinline__ float sample_n_call(const float* __restrict__ a, const NbConst& C, float px, float py, float pz) {
+    return sample_n(a, C.nx, C.ny, C.nz, px, py, pz, C.dx, C.inv_dx, C.dx_pow2 != 0);
+}
+__device__ __noinline__ int2 ray_range(const NbConst& C, float sx, float sy, float sz, float dxr, float dyr, float dzr) {
+    float t0, t1;
+    nb_box_range(sx, sy, sz, dxr, dyr, dzr, C.bmax, t0, t1);
+    return make_int2(trunc_i(t0 / C.dr_f), min(C.nsteps, trunc_i(t1 / C.dr_f) + 2));
+}
+
+// cast_ray with one lane per ray, as a plain loop, where nb_rays_small allows it: the same bits (the
+// products and sums are spelled out where a contraction would change them).  Along the part of the ray
+// that lies a cell inside the box, [i0, i1], the eight corners lie at fixed steps from the lower one, and
+// neither a clamp nor a test of the domain is needed; the half cell to spare is far above the rounding of
+// i0 and i1, which may be approximate.  floor(g) is g added to 1.5 x 2^23 rounded down, whose bits also
+// hold the index: no conversion instruction (those issue at an eighth of the rate).  Samples before i0 and
+// after i1 are sample_n's.  A star inside that part starts at sample 0, so a ray that ends within it never
+// needs its exact range, which costs eight divisions.
+// Issue bound (72% of the slots; 484 instructions a warp at 256^3 with six stars and 512 x 1024 rays), the
+// gathers' cache lines next (51%).  cast_rays with the march over sample_n in 32 rays along phi -> this:
+// 59 -> 35 us at 64^3, 105 -> 60 at 192^3, 118 -> 64 at 256^3; exact build 69 -> 38, 88 -> 48 at 128^3,
+// 126 -> 76 at 192^3.  Two samples at a time (loads of both in flight) measured 8% slower, the clamped form
+// of the corners everywhere 13% slower.
+__device__ __forceinline__ float cast_ray1(const NbConst& C, const float4 d, const float* __restrict__ rho, float sx,
+                                           float sy, float sz, float Q) {
+    const float dr = C.dr_f, dx = C.dx;
+    const float o[3] = {sx, sy, sz}, v[3] = {d.x, d.y, d.z};
+    float i0 = 0.0f, i1 = 1e9f;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const float w = rcp_approx(v[a]), ta = (dx - o[a]) * w, tb = ((C.bmax[a] - dx) - o[a]) * w;
+        i0 = fmaxf(i0, fminf(ta, tb));
+        i1 = fminf(i1, fmaxf(ta, tb));
     }
-    __device__ __forceinline__ float operator()(float gx, float gy, float gz) const {
-        const float M = 12582912.0f;
-        const float mx = fminf(fmaxf(gx - 0.5f, -0.5f), hx) + M, my = fminf(fmaxf(gy - 0.5f, -0.5f), hy) + M;
-        const float mz = fminf(fmaxf(gz - 0.5f, -0.5f), hz) + M;
-        const float fx = __saturatef(gx - (mx - M)), fy = __saturatef(gy - (my - M)), fz = __saturatef(gz - (mz - M));
+    // a star that is no number (every position of its rays is none either) stays with sample_n
+    if (!(fabsf(sx) + fabsf(sy) + fabsf(sz) < 1e30f)) i1 = -1.0f;
+    const bool inside = i0 == 0.0f && i1 > 0.0f;
+    const float inv_dr = rcp_approx(dr);
+    float nf = 0.5f, end = (float)C.nsteps;              // n + 1/2 (exact: nb_rays_small)
+    float sum = 0.0f, comp = 0.0f, rf = C.diag_f;        // Kahan-compensated column
+    auto crosses = [&](float nv, float r) -> bool {
+        const float inc = vmul(vmul(vmul(vmul(nv, nv), r), r), dr), col = sum - comp;
+        if (vadd(col, inc) > Q) {
+            rf = fmaf(-0.5f, dr, r) + dr * (Q - col) / fmaxf(inc, 1e-20f);
+            return true;
+        }
+        const float y = vsub(inc, comp), t = sum + y;
+        comp = (t - sum) - y;
+        sum = t;
+        return false;
+    };
+    auto by_call = [&](float r) {
+        return sample_n_call(rho, C, mac(d.x, r, sx), mac(d.y, r, sy), mac(d.z, r, sz));
+    };
+    if (!inside) {
+        const int2 n = ray_range(C, sx, sy, sz, d.x, d.y, d.z);
+        nf = (float)n.x + 0.5f;
+        end = (float)n.y;
+        for (const float in0 = i0 * inv_dr; nf < end && !(nf >= in0); nf += 1.0f) {
+            const float r = vmul(nf, dr);
+            if (crosses(by_call(r), r)) return rf;
+        }
+    }
+    const float inv_dx = C.inv_dx, M = 12582912.0f, in1 = fminf(i1 * inv_dr, end);
+    const bool pow2 = C.dx_pow2 != 0;
+    const int ny = C.ny, nz = C.nz, sx1 = ny * nz;
+    const unsigned Mb = 0x4B400000u, k = (Mb * (unsigned)ny + Mb) * (unsigned)nz + Mb;   // the bits of M in an index
+    for (; nf < in1; nf += 1.0f) {
+        const float r = vmul(nf, dr), px = mac(d.x, r, sx), py = mac(d.y, r, sy), pz = mac(d.z, r, sz);
+        float gx, gy, gz;
+        if (pow2) {                                      // an exact product
+            gx = fmaf(px, inv_dx, -0.5f);
+            gy = fmaf(py, inv_dx, -0.5f);
+            gz = fmaf(pz, inv_dx, -0.5f);
+        } else {                                         // the quotient is rounded before the subtraction
+            gx = vadd(px / dx, -0.5f);
+            gy = vadd(py / dx, -0.5f);
+            gz = vadd(pz / dx, -0.5f);
+        }
+        const float mx = __fadd_rd(gx, M), my = __fadd_rd(gy, M), mz = __fadd_rd(gz, M);
+        const float fx = gx - (mx - M), fy = gy - (my - M), fz = gz - (mz - M);
         const unsigned e = (__float_as_uint(mx) * (unsigned)ny + __float_as_uint(my)) * (unsigned)nz +
-                           __float_as_uint(mz) - k;
-        const float *p00 = base + e, *p01 = p00 + sy, *p10 = p00 + sx, *p11 = p10 + sy;
+                           (__float_as_uint(mz) - k);
+        const float *p00 = rho + e, *p01 = p00 + nz, *p10 = p00 + sx1, *p11 = p10 + nz;
+#if NB_ARITH_FAST
         const F2 a0 = mk2(__ldg(p00), __ldg(p00 + 1)), a1 = mk2(__ldg(p10), __ldg(p10 + 1));
         const F2 b0 = mk2(__ldg(p01), __ldg(p01 + 1)), b1 = mk2(__ldg(p11), __ldg(p11 + 1));
         const F2 x2 = mk2(fx, fx), y2 = mk2(fy, fy);
         const F2 a = vfma(vsub(a1, a0), x2, a0), b = vfma(vsub(b1, b0), x2, b0), c = vfma(vsub(b, a), y2, a);
-        return fmaf(hi(c) - lo(c), fz, lo(c));
+        const float c0 = lo(c), c1 = hi(c);
+#else
+        const float a0 = __ldg(p00), a1 = __ldg(p10), b0 = __ldg(p01), b1 = __ldg(p11);
+        const float A0 = __ldg(p00 + 1), A1 = __ldg(p10 + 1), B0 = __ldg(p01 + 1), B1 = __ldg(p11 + 1);
+        const float a = mac(a1 - a0, fx, a0), b = mac(b1 - b0, fx, b0), c0 = mac(b - a, fy, a);
+        const float A = mac(A1 - A0, fx, A0), B = mac(B1 - B0, fx, B0), c1 = mac(B - A, fy, A);
+#endif
+        if (crosses(mac(vsub(c1, c0), fz, c0), r)) return rf;
     }
-};
-
-// nebula3d.py:247-270 cast_rays, one lane per ray, on a grid of fewer than 2^31 cells: the march takes
-// only the samples inside the box (outside it the density is 0: they add nothing), so no sample is
-// tested against the domain.
-__device__ __forceinline__ float cast_ray1(const NbConst& C, const float4 d, const float* __restrict__ rho, float sx,
-                                           float sy, float sz, float Q) {
-    const float dr = C.dr_f;
-    float t0 = 0.0f, t1 = 1e9f;
-    const float o[3] = {sx, sy, sz}, dd[3] = {d.x, d.y, d.z};
-    // the box as sample_n's float32 test of p / dx - 1/2 sees it: a position rounds onto a face from half an
-    // ulp outside it (which decides for rays that run in a face)
-    const float e0 = -C.dx * 0x1p-25f, e1 = 1.0f + 0x1p-23f;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {                        // nebula3d.py:229-244 box_range
-        if (fabsf(dd[a]) < 1e-9f) {
-            if (o[a] < 0.0f || o[a] > C.bmax[a]) t1 = -1.0f;
-        } else {
-            const float inv = rcp_approx(dd[a]), ta = (e0 - o[a]) * inv, tb = (C.bmax[a] * e1 - o[a]) * inv;
-            t0 = fmaxf(t0, fminf(ta, tb));
-            t1 = fminf(t1, fmaxf(ta, tb));
-        }
-    }
-    // samples lie at (n + 1/2) dr; n is kept as the float n + 1/2 (exact below 2^23)
-    const float inv_dr = rcp_approx(dr);
-    float nf = fmaxf(ceilf(t0 * inv_dr - 0.5f), 0.0f) + 0.5f;
-    const float n1 = fminf(t1 * inv_dr, (float)C.nsteps - 0.5f);
-    const CellSampler at(C, rho);
-    const float inv_dx = C.dx_pow2 ? C.inv_dx : rcp_approx(C.dx);
-    float sum = 0.0f, comp = 0.0f, rf = C.diag_f;        // Kahan-compensated column
-    for (; nf <= n1; nf += 1.0f) {
-        const float r = nf * dr;
-        // the position first, then in cells, and the product in the reference's order: the fronts are those
-        // of the general form to the bit but where a sample lies on a cell centre or in the outermost half
-        // cell.  (Folding both into one multiply-add moves fronts by 3e-7 of the box, which a stiff front
-        // amplifies to 1e-3 of the momentum in single cells within a few steps.)
-        const float nv = at(fmaf(fmaf(d.x, r, sx), inv_dx, -0.5f), fmaf(fmaf(d.y, r, sy), inv_dx, -0.5f),
-                            fmaf(fmaf(d.z, r, sz), inv_dx, -0.5f));
-        const float inc = nv * nv * r * r * dr, col = sum - comp;
-        if (col + inc > Q) {
-            rf = r - 0.5f * dr + dr * (Q - col) / fmaxf(inc, 1e-20f);
-            break;
-        }
-        const float y = inc - comp, t = sum + y;
-        comp = (t - sum) - y;
-        sum = t;
+    if (inside) end = (float)ray_range(C, sx, sy, sz, d.x, d.y, d.z).y;
+    for (; nf < end; nf += 1.0f) {
+        const float r = vmul(nf, dr);
+        if (crosses(by_call(r), r)) return rf;
     }
     return rf;
-}
-#endif
-
-// The direction (iu, ip) of a star's q-th ray.  A warp takes 8 (u) x 4 (phi) neighbouring directions
-// where the ray grid divides so: the bundle stays within a few cells, so its rays share cache lines and
-// end within a few samples of one another, and its fronts fill whole sectors of the [phi][u] table (32
-// neighbours along phi span an arc ten times as wide).  With CellSampler (225 instead of 380 thread
-// instructions a cell at 192^3): cast_rays 118 -> 78 us at 256^3, 105 -> 69 at 192^3, 59 -> 48 at 64^3;
-// the exact build, whose sampler stays, is level.
-__device__ __forceinline__ int2 ray_dir(int q, int nu, int nphi) {
-    if ((nu & 7) || (nphi & 3)) {
-        const int iu = q / nphi;
-        return make_int2(iu, q - iu * nphi);
-    }
-    const int t = q >> 5, l = q & 31, tu = nu >> 3, tp = t / tu;
-    return make_int2((t - tp * tu) * 8 + (l & 7), tp * 4 + (l >> 3));
 }
 
 // Each star's least and largest front radius, for apply_front's culling: order-preserving bits of the
@@ -277,62 +300,59 @@ __device__ __forceinline__ void merge_front(uint2* bounds, int id, int s, float 
     }
 }
 
-// The front of ray (iu, ip) of star s into an instance's table [star][phi][u]: one float, or (pairs)
+// The front of the ray along d of star s into an instance's table [star][phi][u]: one float, or (pairs)
 // the .x of its own float2 pair and the .y of the pair below it (and of its own at the last u).
-__device__ __forceinline__ void put_front(float* rfront, bool pairs, int s, long long nray, int nu, int iu, int ip,
+__device__ __forceinline__ void put_front(float* rfront, bool pairs, int s, long long nray, int nu, const float4 d,
                                           float rf) {
-    const long long e = (long long)s * nray + (long long)ip * nu + iu;
+    const int w = __float_as_int(d.w);
+    const long long e = (long long)s * nray + (w & 0x7fffffff);
     if (!pairs) {
         rfront[e] = rf;
         return;
     }
     float* p = rfront + 2 * e;
     p[0] = rf;
-    if (iu > 0) p[-1] = rf;
-    if (iu == nu - 1) p[1] = rf;
+    // w < 0: the first u (below 0) or the last (above 0), or both where nu is 1
+    if (w >= 0 || (d.z > 0.0f && nu > 1)) p[-1] = rf;
+    if (w < 0 && (d.z > 0.0f || nu == 1)) p[1] = rf;
 }
 
-// The front radius of direction (iu, ip) of a star.  SMALL: the one-lane form of the fast build.
+// The front radius along d.  SMALL: cast_ray1.
 template <int G, bool SMALL>
-__device__ __forceinline__ float cast_dir(const NbConst& C, const float4* __restrict__ dirs,
-                                          const float* __restrict__ rho, int2 dir, float sx, float sy, float sz, float Q,
-                                          int lane, unsigned gmask, bool live) {
-    const int ray = dir.x * C.nphi + dir.y;
-#if NB_ARITH_FAST
-    if (SMALL) return live ? cast_ray1(C, dirs[ray], rho, sx, sy, sz, Q) : 0.0f;
-#endif
-    return cast_ray<G>(C, dirs, rho, ray, sx, sy, sz, Q, lane, gmask, live);
+__device__ __forceinline__ float cast_dir(const NbConst& C, const float4 d, const float* __restrict__ rho, float sx,
+                                          float sy, float sz, float Q, int lane, unsigned gmask, bool live) {
+    if (SMALL) return live ? cast_ray1(C, d, rho, sx, sy, sz, Q) : 0.0f;
+    return cast_ray<G>(C, d, rho, sx, sy, sz, Q, lane, gmask, live);
 }
 
 // Resident blocks per SM of the ray kernel: 5 (48 registers); at 6 (40 registers) the warp-uniform
 // march spills 44-84 bytes.
 #define NB_CAST_RAYS_MINB 5
+// blockIdx.y: the star
 template <int G, bool PAIRS, bool SMALL>
 __global__ void __launch_bounds__(256, NB_CAST_RAYS_MINB)
     cast_rays_kernel(const NbConst* __restrict__ c, const NbStarW* __restrict__ sw, const float4* __restrict__ dirs,
-                     const float* __restrict__ rho, float* __restrict__ rfront, int nstars, uint2* bounds,
+                     const float* __restrict__ rho, float* __restrict__ rfront, uint2* bounds,
                      const float* star_override, float q_override) {
-    const int nray = c->nu * c->nphi;
+    const int nray = c->nu * c->nphi, s = blockIdx.y;
     const long long gid = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / G;
     const int lane = threadIdx.x % G;
     const unsigned gmask = G == 32 ? 0xffffffffu : (((1u << G) - 1u) << ((threadIdx.x & 31) / G * G));
     // no early exit: every thread reaches the march's warp-wide operations and the merge's barriers
-    const bool in = gid < (long long)nray * nstars;
-    // a group index of one instance stays below 2^32 (nb_create checks it): 32-bit division
-    const unsigned g32 = in ? (unsigned)gid : 0u;
-    const int s = (int)(g32 / (unsigned)nray);
-    const int2 dir = ray_dir((int)(g32 - (unsigned)s * (unsigned)nray), c->nu, c->nphi);
+    const bool in = gid < nray;
+    const float4 d = dirs[in ? (int)gid : 0];
     if (star_override) {
-        const float rf = cast_dir<G, SMALL>(*c, dirs, rho, dir, star_override[0], star_override[1], star_override[2],
+        const float rf = cast_dir<G, SMALL>(*c, d, rho, star_override[0], star_override[1], star_override[2],
                                             q_override, lane, gmask, in);
-        if (in && lane == 0) rfront[dir.x * c->nphi + dir.y] = rf;
+        const int e = __float_as_int(d.w) & 0x7fffffff, ip = e / c->nu;
+        if (in && lane == 0) rfront[(e - ip * c->nu) * c->nphi + ip] = rf;
         return;
     }
     const NbStarW w = sw[s];
     const bool live = in && w.active;
-    const float rf = cast_dir<G, SMALL>(*c, dirs, rho, dir, w.w.x, w.w.y, w.w.z, w.q_f, lane, gmask, live);
+    const float rf = cast_dir<G, SMALL>(*c, d, rho, w.w.x, w.w.y, w.w.z, w.q_f, lane, gmask, live);
     // the instance's table is [star][phi][u] (u fastest: the cells of a warp share phi)
-    if (live && lane == 0) put_front(rfront, PAIRS, s, nray, c->nu, dir.x, dir.y, rf);
+    if (live && lane == 0) put_front(rfront, PAIRS, s, nray, c->nu, d, rf);
     if (bounds) merge_front(bounds, s, s, rf, live);
 }
 
@@ -359,13 +379,13 @@ __device__ __forceinline__ void cast_rays_batch_body(const Jobs& J, const NbRayJ
     const long long local = gid - job.ray0;
     const unsigned l32 = (unsigned)local;        // below 2^32 within a job (nb_create): 32-bit division
     const int s = (int)(l32 / (unsigned)nray);
-    const int2 dir = ray_dir((int)(l32 - (unsigned)s * (unsigned)nray), C.nu, C.nphi);
+    const float4 d = job.dirs[l32 - (unsigned)s * (unsigned)nray];
     const bool star = in && s < job.nstars && Jd[lo].active;
     NbStarW w{};
     if (star) w = job.sw[s];
     const bool live = star && w.active;
-    const float rf = cast_dir<G, SMALL>(C, job.dirs, job.rho, dir, w.w.x, w.w.y, w.w.z, w.q_f, lane, gmask, live);
-    if (live && lane == 0) put_front(job.rfront, job.pairs != 0, s, nray, C.nu, dir.x, dir.y, rf);
+    const float rf = cast_dir<G, SMALL>(C, d, job.rho, w.w.x, w.w.y, w.w.z, w.q_f, lane, gmask, live);
+    if (live && lane == 0) put_front(job.rfront, job.pairs != 0, s, nray, C.nu, d, rf);
     // the lanes of a warp may belong to two jobs: (job, star) pairs are told apart
     merge_front(job.front_bounds, lo * NB_MAX_STARS + s, s, rf, live && job.front_bounds);
 }
@@ -730,19 +750,34 @@ cudaError_t nb_launch_ray_dirs(int nu, int nphi, float4* dirs, cudaStream_t s) {
     return cudaGetLastError();
 }
 
+cudaError_t nb_launch_ray_order(int nu, int nphi, const float4* dirs, float4* out, cudaStream_t s) {
+    const int n = nu * nphi;
+    ray_order_kernel<<<(n + 255) / 256, 256, 0, s>>>(nu, nphi, dirs, out);
+    return cudaGetLastError();
+}
+
+// cast_ray1's rule, on the host: cells, samples and the index of a corner are exact in its floats and
+// 32-bit integers, the part of the box a cell from its faces is there, and the cell size keeps every
+// product and quotient of positions normal.
+int nb_rays_small(const NbConst& c) {
+    const int most = 1 << 16;
+    return c.nx >= 4 && c.ny >= 4 && c.nz >= 4 && c.nx <= most && c.ny <= most && c.nz <= most &&
+           (long long)c.nx * c.ny * c.nz < (1LL << 31) && c.nsteps <= (1 << 22) && c.dx > 1e-12f && c.dx < 1e12f;
+}
+
 cudaError_t nb_launch_cast_rays(const NbConst* c, const NbStarW* sw, const float4* dirs, const float* rho,
                                 float* rfront, int nstars, int group, uint2* bounds, const float* star_override,
                                 float q_override, cudaStream_t s, int nu, int nphi, int pairs, int small) {
-    const long long threads = (long long)nu * nphi * nstars * group;
-    const int blocks = (int)((threads + 255) / 256);
+    const long long threads = (long long)nu * nphi * group;
+    const dim3 blocks((unsigned)((threads + 255) / 256), (unsigned)nstars);
 #define NB_RAYS_LAUNCH(G, SM)                                                                                      \
-    (pairs ? cast_rays_kernel<G, true, SM><<<blocks, 256, 0, s>>>(c, sw, dirs, rho, rfront, nstars, bounds,         \
+    (pairs ? cast_rays_kernel<G, true, SM><<<blocks, 256, 0, s>>>(c, sw, dirs, rho, rfront, bounds, \
                                                                   star_override, q_override)                        \
-           : cast_rays_kernel<G, false, SM><<<blocks, 256, 0, s>>>(c, sw, dirs, rho, rfront, nstars, bounds,        \
+           : cast_rays_kernel<G, false, SM><<<blocks, 256, 0, s>>>(c, sw, dirs, rho, rfront, bounds,                \
                                                                    star_override, q_override))
     switch (group) {
         case 1:
-            if (NB_RAYS_SMALL && small) NB_RAYS_LAUNCH(1, NB_RAYS_SMALL);
+            if (small) NB_RAYS_LAUNCH(1, true);
             else NB_RAYS_LAUNCH(1, false);
             break;
         case 2: NB_RAYS_LAUNCH(2, false); break;
@@ -790,8 +825,8 @@ cudaError_t nb_launch_ionize_batch(const NbRayJob* jobs, const NbRayJob* host_jo
         const unsigned nb = (unsigned)blocks;
         switch (group) {
             case 1:
-                if (NB_RAYS_SMALL && small)
-                    cast_rays_batch_param_kernel<1, NB_RAYS_SMALL><<<nb, 256, 0, s>>>(P, jobs, n_jobs, n_groups);
+                if (small)
+                    cast_rays_batch_param_kernel<1, true><<<nb, 256, 0, s>>>(P, jobs, n_jobs, n_groups);
                 else
                     cast_rays_batch_param_kernel<1, false><<<nb, 256, 0, s>>>(P, jobs, n_jobs, n_groups);
                 break;
@@ -804,8 +839,8 @@ cudaError_t nb_launch_ionize_batch(const NbRayJob* jobs, const NbRayJob* host_jo
     } else if (blocks > 0) {
         switch (group) {
             case 1:
-                if (NB_RAYS_SMALL && small)
-                    cast_rays_batch_kernel<1, NB_RAYS_SMALL><<<(unsigned)blocks, 256, 0, s>>>(jobs, n_jobs, n_groups);
+                if (small)
+                    cast_rays_batch_kernel<1, true><<<(unsigned)blocks, 256, 0, s>>>(jobs, n_jobs, n_groups);
                 else
                     cast_rays_batch_kernel<1, false><<<(unsigned)blocks, 256, 0, s>>>(jobs, n_jobs, n_groups);
                 break;
