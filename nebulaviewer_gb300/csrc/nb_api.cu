@@ -26,7 +26,7 @@ struct nb_instance {
     float4* dirs = nullptr;             // ionizing-ray directions (nu * nphi)
     float4* dirs_fuv = nullptr;         // FUV-ray directions (fnu * fnphi)
     float* rfront = nullptr;            // [star][nphi][nu] (float2 (u, u + 1) pairs with front_pairs)
-    float* att = nullptr;               // [star][fnu][fnphi][fnr] (float2 (r, r + 1) pairs with fuv_pairs)
+    float* att = nullptr;               // per star fnu * fnphi * fnr entries, float2 (r, r + 1) pairs with fuv_pairs (nb_fuv.cu)
     float* scratch3 = nullptr;          // 3 floats: a single star position for the one-star kernels
     float* plane_xf = nullptr;          // [ny][nz] front of the -x plane source
     double* red = nullptr;              // FP64 reduction partials
@@ -763,7 +763,7 @@ NB_EXPORT int nb_fuv(nb_handle h) {
         Prof pf(h, NB_PROF_CAST_FUV, 2);                // the (rho, xi) pack into stage planes 0-1 + the rays
         CK(h, nb_launch_cast_fuv(h->c, h->sw, h->dirs_fuv, h->d.f.rho, h->d.f.xi, h->att, h->nstars, h->fuv_group,
                                  nullptr, 0, h->stream, h->d.fnu, h->d.fnphi, plane(h, 0), h->ncell,
-                                 h->fuv_cut ? NB_FUV_TAU_CUT : 0.0f, h->fuv_pairs));
+                                 h->fuv_cut ? NB_FUV_TAU_CUT : 0.0f, h->fuv_pairs, h->d.fnr));
     }
     if (h->hc.plane_on) {
         Prof pf(h, NB_PROF_CAST_FUV, 1);
@@ -772,7 +772,7 @@ NB_EXPORT int nb_fuv(nb_handle h) {
     {
         Prof pf(h, NB_PROF_APPLY_FUV, 1);
         CK(h, nb_launch_apply_fuv(h->c, h->sw, h->att, h->nstars, h->d.f.g0, h->stream, h->d.nx,
-                                  h->d.ny, h->d.fields_fp32 ? 0 : 1, h->fuv_pairs));
+                                  h->d.ny, h->d.fields_fp32 ? 0 : 1, h->fuv_pairs, h->d.fnr, h->d.fnu));
     }
     return NB_OK;
 }
@@ -823,7 +823,7 @@ NB_EXPORT int nb_cast_fuv(nb_handle h, const double xyz[3], float* att_out) {
     CK(h, cudaMemcpyAsync(h->scratch3, s3, sizeof(s3), cudaMemcpyHostToDevice, h->stream));
     CK(h, nb_launch_cast_fuv(h->c, h->sw, h->dirs_fuv, h->d.f.rho, h->d.f.xi, att_out, 1, 32, h->scratch3, 1,
                              h->stream, h->d.fnu, h->d.fnphi, plane(h, 0), h->ncell, h->fuv_cut ? NB_FUV_TAU_CUT : 0.0f,
-                             0));
+                             0, h->d.fnr));
     CK(h, cudaStreamSynchronize(h->stream));
     return NB_OK;
 }

@@ -6,15 +6,23 @@
 // GB300 design: cast_fuv marches a ray with a group of G lanes, the optical depth being an
 // inclusive group scan over a Kahan-compensated carry; a lane that crosses into new radial
 // bins writes them, and a ray stops once its optical depth passes 120 (exp(-tau) is 0.0f from
-// there on: its remaining bins are written as 0).  Density and ionized fraction are sampled at the same corners, so they
-// are first packed as (rho, xi) pairs into free scratch: one 8-byte gather per corner.  All rays of all active stars are one launch, into one attenuation grid
-// per star laid out [star][u][phi][r] (r fastest: a ray's bins are contiguous).  Each entry is
-// the pair (att(r), att(min(r + 1, nr - 1))) as one float2 (the ray writes each bin into its own
-// pair and its lower neighbour's), so a trilinear sample of apply_fuv is four 8-byte gathers
+// there on: its remaining bins are written as 0).  Density and ionized fraction are sampled at the
+// same corners, so they are first packed as (rho, xi) pairs into free scratch: one 8-byte gather per
+// corner.  All rays of all active stars are one launch, into one attenuation table per star.  An
+// entry is the pair (att(r), att(min(r + 1, nr - 1))) as one float2 (the ray writes each bin into
+// its own pair and its lower neighbour's), so a trilinear sample of apply_fuv is four 8-byte gathers
 // instead of eight 4-byte ones; values and arithmetic are those of the plain table
-// (NB_TUNE_FUV_PAIRS = 0), bit for bit.  apply_fuv accumulates every active star for a cell in
-// one register, in the reference's star order (so the float32 sum is the reference's), and
-// stores G0 once as fp16.
+// (NB_TUNE_FUV_PAIRS = 0), bit for bit, in whichever order the entries lie.  apply_fuv accumulates
+// every active star for a cell in one register, in the reference's star order (so the float32 sum
+// is the reference's), and stores G0 once as fp16.
+//
+// Both kernels were bound by L1 wavefronts (a gather takes one per 128-byte line it touches).  The
+// table lies in bricks of 4 u x 4 r, one line each (a ray still writes whole 32-byte sectors), the
+// rays of a brick are cast together, and a warp of the apply takes 4 x 2 x 4 cells instead of 32
+// along k: 21 lines per cell group and star instead of 48.  apply_fuv at 64^3 / 192^3 / 256^3 /
+// 384^3 with six stars: 30 / 256 / 563 / 1954 -> 18 / 177 / 395 / 1298 us (cells alone 458 at
+// 256^3), now issue bound (88%); cast_fuv with its pack 630 -> 590 us at 256^3 (whole pairs where
+// a ray fills its last bins), level below 128^3.
 #include "nb_rayutil.cuh"
 
 namespace {
@@ -25,7 +33,28 @@ __global__ void __launch_bounds__(256) pack_rx_kernel(const float* __restrict__ 
         rx[q] = make_float2(rho[q], xi[q]);
 }
 
-template <int G, bool REF_LAYOUT, bool PAIRS>
+// Layouts of an instance's attenuation table, per star.
+enum {
+    FUV_PLAIN,      // [u][phi][r], one float
+    FUV_PAIRS,      // [u][phi][r], (att(r), att(min(r + 1, nr - 1)))
+    FUV_BRICKS,     // the pairs, [phi][u / 4][r / 4][u % 4][r % 4]: a 128-byte line holds 4 u x 4 r
+    FUV_REF         // [r][u][phi], one float (a cast into the caller's array)
+};
+// An entry's offset is the sum of three: of its phi, its u and its r.
+template <int L>
+__device__ __forceinline__ int fuv_phi(int ip, int nu, int nr) {
+    return ip * (L == FUV_BRICKS ? nu * nr : nr);
+}
+template <int L>
+__device__ __forceinline__ int fuv_u(int iu, int nphi, int nr) {
+    return L == FUV_BRICKS ? 4 * iu + (iu >> 2) * (4 * nr - 16) : iu * (nphi * nr);
+}
+template <int L>
+__device__ __forceinline__ int fuv_r(int ir) {
+    return L == FUV_BRICKS ? ir + 12 * (ir >> 2) : ir;
+}
+
+template <int G, int L>
 __global__ void __launch_bounds__(256, 5) cast_fuv_kernel(const NbConst* __restrict__ c, const NbStarW* __restrict__ sw,
                                                        const float4* __restrict__ dirs,
                                                        const float2* __restrict__ rx,
@@ -46,26 +75,37 @@ __global__ void __launch_bounds__(256, 5) cast_fuv_kernel(const NbConst* __restr
         if (!w.active) return;
         sx = w.w.x; sy = w.w.y; sz = w.w.z;
     }
-    const int iu = ray / nphi, ip = ray % nphi;
-    // bin b of this ray: the reference layout [b][iu][ip], or the instance's [star][u][phi][b] (a ray's
-    // bins contiguous; a u-fastest layout makes the apply's gathers contiguous but scatters these writes,
-    // a net loss measured at 256^3)
+    // bricks: four u in turn, so that the rays of a line of the table are cast together
+    const int iu = L == FUV_BRICKS ? ray / (4 * nphi) * 4 + (ray & 3) : ray / nphi;
+    const int ip = L == FUV_BRICKS ? (ray >> 2) % nphi : ray % nphi;
+    float* const table = L == FUV_REF ? att : att + (L == FUV_PLAIN ? 1 : 2) * ((long long)s * nray * nr);
+    const int at = fuv_phi<L>(ip, nu, nr) + fuv_u<L>(iu, nphi, nr);
     auto put = [&](int b, float v) {
-        if (REF_LAYOUT) {
+        if (L == FUV_REF) {
             att[((long long)b * nu + iu) * nphi + ip] = v;
-        } else if (!PAIRS) {
-            att[((long long)s * nray + ray) * nr + b] = v;
+        } else if (L == FUV_PLAIN) {
+            table[at + b] = v;
         } else {                                 // bin b is pair b's .x and pair b-1's .y
-            float* p = att + 2 * (((long long)s * nray + ray) * nr + b);
-            p[0] = v;
-            if (b > 0) p[-1] = v;
-            if (b == nr - 1) p[1] = v;
+            float* p = table + 2 * (long long)at;
+            p[2 * fuv_r<L>(b)] = v;
+            if (b > 0) p[2 * fuv_r<L>(b - 1) + 1] = v;
+            if (b == nr - 1) p[2 * fuv_r<L>(b) + 1] = v;
+        }
+    };
+    // every bin from b0 on: whole pairs
+    auto fill = [&](int b0, float v) {
+        if (L == FUV_REF || L == FUV_PLAIN) {
+            for (int b = b0 + lane; b < nr; b += G) put(b, v);
+        } else {
+            float2* p = reinterpret_cast<float2*>(table) + at;
+            for (int b = b0 + lane; b < nr; b += G) p[fuv_r<L>(b)] = make_float2(v, v);
+            if (lane == 0 && b0 > 0 && b0 < nr) p[fuv_r<L>(b0 - 1)].y = v;
         }
     };
     const int nx = c->nx, ny = c->ny, nz = c->nz;
     const float dx = c->dx, inv_dx = c->inv_dx, dr = c->dr_f, binr = c->binr_f, kappa = c->kappa_f;
     const bool pow2 = c->dx_pow2 != 0;
-    const float4 d = dirs[ray];
+    const float4 d = dirs[iu * nphi + ip];
     float t0, t1;
     nb_box_range(sx, sy, sz, d.x, d.y, d.z, c->bmax, t0, t1);
     const int n0 = trunc_i(t0 / dr);
@@ -109,7 +149,7 @@ __global__ void __launch_bounds__(256, 5) cast_fuv_kernel(const NbConst* __restr
         }
         if (mine) {                              // a lane ran out of bins or into the dark
             const int e_first = __shfl_sync(gmask, min(nb, nr), first_stop, G);
-            for (int b = e_first + lane; b < nr; b += G) put(b, 0.0f);
+            fill(e_first, 0.0f);
             stopped = true;
             break;
         }
@@ -121,20 +161,17 @@ __global__ void __launch_bounds__(256, 5) cast_fuv_kernel(const NbConst* __restr
         comp = (tsum - hi) - y;
         hi = tsum;
     }
-    if (!stopped) {
-        const float v = expf(-(hi - comp));
-        for (int b = ib + lane; b < nr; b += G) put(b, v);
-    }
+    if (!stopped) fill(ib, expf(-(hi - comp)));
 }
 
-template <bool HALF, bool PAIRS>
+template <bool HALF, int L>
 __global__ void __launch_bounds__(256, 6) apply_fuv_kernel(const NbConst* __restrict__ c, const NbStarW* __restrict__ sw,
                                                         const float* __restrict__ att, int nstars,
-                                                        void* __restrict__ g0) {
+                                                        void* __restrict__ g0, int li) {
     __shared__ float4 st[NB_MAX_STARS];
     __shared__ float lum[NB_MAX_STARS];
     __shared__ int act[NB_MAX_STARS];
-    __shared__ float4 rowtab[8][NB_ROW_STARS];
+    __shared__ float4 rowtab[8][NB_ROW_STARS + 1];       // + 1: the eight rows of a warp in different banks
     for (int s = threadIdx.y * blockDim.x + threadIdx.x; s < nstars; s += blockDim.x * blockDim.y) {
         st[s] = sw[s].w;
         lum[s] = sw[s].lum_f;
@@ -144,28 +181,29 @@ __global__ void __launch_bounds__(256, 6) apply_fuv_kernel(const NbConst* __rest
     const int nx = c->nx, ny = c->ny, nz = c->nz, nr = c->fnr, nu = c->fnu, nphi = c->fnphi;
     const float dx = c->dx, binr = c->binr_f;
     const float two_pi = 2.0f * pi_f();
+    const int colmul = fuv_phi<L>(1, nu, nr);   // offsets within a star's table are below 2^31
     const int C_plane_on = c->plane_on;
     const float* C_plane_g0 = c->plane_g0;
-    const RowWalk w(nx, ny, nz);
-    if (!w.valid) return;
-    const float px = ((float)w.i + 0.5f) * dx, py = ((float)w.j + 0.5f) * dx;
+    // a block takes 2^li x 2^lj rows, a warp 4 cells of each of them at a time
+    const int lj = 3 - li, nbj = (ny + (1 << lj) - 1) >> lj, bi = blockIdx.x / nbj, bj = blockIdx.x - bi * nbj;
     // per-row azimuth constants (star_row_table): the same values the per-cell form computes
-    float4* tab = nstars <= NB_ROW_STARS ? rowtab[threadIdx.y] : nullptr;
-    if (tab) star_row_table(st, act, nstars, px, py, nphi, 1, tab);
-    for (int k = w.k0; k < nz; k += 32) {
-        const long long q = w.base + k;
+    float4* tab = nullptr;
+    if (nstars <= NB_ROW_STARS) {
+        const int r = threadIdx.y, i = (bi << li) + (r >> lj), j = (bj << lj) + (r & ((1 << lj) - 1));
+        star_row_table(st, act, nstars, ((float)i + 0.5f) * dx, ((float)j + 0.5f) * dx, nphi, colmul, rowtab[r]);
+        __syncthreads();
+        tab = rowtab[threadIdx.x >> 2];
+    }
+    const int row = threadIdx.x >> 2, wi = (bi << li) + (row >> lj), wj = (bj << lj) + (row & ((1 << lj) - 1));
+    if (wi >= nx || wj >= ny) return;
+    const float px = ((float)wi + 0.5f) * dx, py = ((float)wj + 0.5f) * dx;
+    const long long base = ((long long)wi * ny + wj) * nz;
+    for (int k = threadIdx.y * 4 + (threadIdx.x & 3); k < nz; k += 32) {
+        const long long q = base + k;
         const float pz = ((float)k + 0.5f) * dx;
         float g = 0.0f;
-        constexpr int SG = 2;                    // stars whose gathers are in flight together
-        for (int s0 = 0; s0 < nstars; s0 += SG) {
-          float term[SG];
-          bool on[SG];
-#pragma unroll
-          for (int e = 0; e < SG; ++e) {
-            const int s = s0 + e;
-            on[e] = s < nstars && act[s];
-            term[e] = 0.0f;
-            if (!on[e]) continue;
+        for (int s = 0; s < nstars; ++s) {
+            if (!act[s]) continue;
             const float4 sp = st[s];
             const float rz = pz - sp.z;
             float r, tp;
@@ -184,27 +222,28 @@ __global__ void __launch_bounds__(256, 6) apply_fuv_kernel(const NbConst* __rest
                 const float fp = phi / two_pi * (float)nphi - 0.5f;
                 const int ip = (int)floorf(fp);
                 tp = fp - (float)ip;
-                pw[0] = wrap_index(ip, nphi);
-                pw[1] = wrap_index(ip + 1, nphi);
+                pw[0] = wrap_index(ip, nphi) * colmul;
+                pw[1] = wrap_index(ip + 1, nphi) * colmul;
             }
             const float u = rz / r;
             const float fr = r / binr - 0.5f;
             const float fu = (u + 1.0f) * 0.5f * (float)nu - 0.5f;
-            const int ir = (int)floorf(fr), iu = (int)floorf(fu);
-            const float tr = fr - (float)ir, tu = fu - (float)iu;
+            const float flr = floorf(fr), flu = floorf(fu);
+            const int ir = (int)flr, iu = (int)flu;
+            const float tr = fr - flr, tu = fu - flu;
             const long long tab0 = (long long)s * nu * nphi * nr;
+            const int ua = fuv_u<L>(iclampd(iu, 0, nu - 1), nphi, nr), ub = fuv_u<L>(iclampd(iu + 1, 0, nu - 1), nphi, nr);
             float v[2][2][2];                    // [r corner][u corner][phi corner]
-            if (PAIRS) {
+            if (L != FUV_PLAIN) {
                 // pair rc = (att(rc), att(min(rc + 1, nr - 1))): the two r corners, except at ir = -1,
                 // where both clamp to r = 0 (the pair's .x)
                 const float2* ap = reinterpret_cast<const float2*>(att) + tab0;
-                const int rc = iclampd(ir, 0, nr - 1);
+                const int rc = fuv_r<L>(iclampd(ir, 0, nr - 1));
 #pragma unroll
                 for (int bb = 0; bb < 2; ++bb)
 #pragma unroll
                     for (int cc = 0; cc < 2; ++cc) {
-                        const int uu = iclampd(iu + bb, 0, nu - 1);
-                        const float2 pr = __ldg(ap + ((uu * nphi + pw[cc]) * nr + rc));      // < 2^31 per star
+                        const float2 pr = __ldg(ap + ((bb ? ub : ua) + pw[cc] + rc));
                         v[0][bb][cc] = pr.x;
                         v[1][bb][cc] = ir < 0 ? pr.x : pr.y;
                     }
@@ -217,8 +256,7 @@ __global__ void __launch_bounds__(256, 6) apply_fuv_kernel(const NbConst* __rest
 #pragma unroll
                         for (int cc = 0; cc < 2; ++cc) {
                             const int rr = iclampd(ir + aa, 0, nr - 1);
-                            const int uu = iclampd(iu + bb, 0, nu - 1);
-                            v[aa][bb][cc] = __ldg(as + ((uu * nphi + pw[cc]) * nr + rr));   // < 2^31 per star
+                            v[aa][bb][cc] = __ldg(as + ((bb ? ub : ua) + pw[cc] + rr));
                         }
             }
             float acc = 0.0f;
@@ -232,11 +270,8 @@ __global__ void __launch_bounds__(256, 6) apply_fuv_kernel(const NbConst* __rest
                         acc = acc + wgt * v[aa][bb][cc];
                     }
             const float r2 = fmaxq(r * r, 0.0004f);
-            term[e] = lum[s] * acc / r2;
-          }
-#pragma unroll
-          for (int e = 0; e < SG; ++e)
-            if (on[e]) g = g + term[e];                 // the reference's star order
+            const float term = lum[s] * acc / r2;      // rounded before the sum in both builds
+            g = __fadd_rn(g, term);                     // the reference's star order
         }
         if (C_plane_on) g = g + __ldg(C_plane_g0 + q);      // the -x plane source, after the stars
         if (HALF)
@@ -273,10 +308,14 @@ cudaError_t nb_launch_plane_fuv(const NbConst* c, const float* rho, const float*
     return cudaGetLastError();
 }
 
+// Bricks where they need no padding: a table is then as large as in the other orders.  (Every ray
+// budget a simulation chooses for itself is a multiple of 4.)
+static bool fuv_bricks(int fnr, int fnu) { return fnr % 4 == 0 && fnu % 4 == 0; }
+
 cudaError_t nb_launch_cast_fuv(const NbConst* c, const NbStarW* sw, const float4* dirs, const float* rho,
                                const float* xi, float* att, int nstars, int group, const float* star_override,
                                int ref_layout, cudaStream_t s, int fnu, int fnphi, void* rx_scratch, long long ncell,
-                               float tau_cut, int pairs) {
+                               float tau_cut, int pairs, int fnr) {
     float2* rx = static_cast<float2*>(rx_scratch);
     {
         const long long b = (ncell + 255) / 256;
@@ -284,37 +323,42 @@ cudaError_t nb_launch_cast_fuv(const NbConst* c, const NbStarW* sw, const float4
     }
     const long long threads = (long long)fnu * fnphi * nstars * group;
     const int blocks = (int)((threads + 255) / 256);
-#define NB_FUV_LAUNCH(G, R, PR) \
-    cast_fuv_kernel<G, R, PR><<<blocks, 256, 0, s>>>(c, sw, dirs, rx, att, nstars, star_override, tau_cut)
-    if (ref_layout) {
-        NB_FUV_LAUNCH(32, true, false);
-    } else if (pairs) {
-        switch (group) {
-            case 8: NB_FUV_LAUNCH(8, false, true); break;
-            case 16: NB_FUV_LAUNCH(16, false, true); break;
-            default: NB_FUV_LAUNCH(32, false, true); break;
-        }
-    } else {
-        switch (group) {
-            case 8: NB_FUV_LAUNCH(8, false, false); break;
-            case 16: NB_FUV_LAUNCH(16, false, false); break;
-            default: NB_FUV_LAUNCH(32, false, false); break;
-        }
+#define NB_FUV_LAUNCH(G, L) \
+    cast_fuv_kernel<G, L><<<blocks, 256, 0, s>>>(c, sw, dirs, rx, att, nstars, star_override, tau_cut)
+#define NB_FUV_GROUPS(L)                          \
+    switch (group) {                              \
+        case 8: NB_FUV_LAUNCH(8, L); break;       \
+        case 16: NB_FUV_LAUNCH(16, L); break;     \
+        default: NB_FUV_LAUNCH(32, L); break;     \
     }
+    if (ref_layout) {
+        NB_FUV_LAUNCH(32, FUV_REF);
+    } else if (pairs && fuv_bricks(fnr, fnu)) {
+        NB_FUV_GROUPS(FUV_BRICKS)
+    } else if (pairs) {
+        NB_FUV_GROUPS(FUV_PAIRS)
+    } else {
+        NB_FUV_GROUPS(FUV_PLAIN)
+    }
+#undef NB_FUV_GROUPS
 #undef NB_FUV_LAUNCH
     return cudaGetLastError();
 }
 
 cudaError_t nb_launch_apply_fuv(const NbConst* c, const NbStarW* sw, const float* att, int nstars, void* g0,
-                                cudaStream_t s, int nx, int ny, int half, int pairs) {
-    const int blocks = rowwalk_blocks(nx, ny);
-    if (half && pairs)
-        apply_fuv_kernel<true, true><<<blocks, dim3(32, 8), 0, s>>>(c, sw, att, nstars, g0);
-    else if (half)
-        apply_fuv_kernel<true, false><<<blocks, dim3(32, 8), 0, s>>>(c, sw, att, nstars, g0);
-    else if (pairs)
-        apply_fuv_kernel<false, true><<<blocks, dim3(32, 8), 0, s>>>(c, sw, att, nstars, g0);
-    else
-        apply_fuv_kernel<false, false><<<blocks, dim3(32, 8), 0, s>>>(c, sw, att, nstars, g0);
+                                cudaStream_t s, int nx, int ny, int half, int pairs, int fnr, int fnu) {
+    // 4 x 2 rows a block, or another split where that leaves far more lanes without a row (thin and small
+    // grids): 2 x 4 and 1 x 8 rows took 10% longer at 192^3 and 256^3
+    int li = 2, blocks = ((nx + 3) / 4) * ((ny + 1) / 2);
+    const int b2 = ((nx + 1) / 2) * ((ny + 3) / 4), b1 = nx * ((ny + 7) / 8);
+    if (b2 < blocks - blocks / 10) li = 1, blocks = b2;
+    if (b1 < blocks - blocks / 10) li = 0, blocks = b1;
+#define NB_FUV_APPLY(L)                                                                                   \
+    (half ? apply_fuv_kernel<true, L><<<blocks, dim3(32, 8), 0, s>>>(c, sw, att, nstars, g0, li)          \
+          : apply_fuv_kernel<false, L><<<blocks, dim3(32, 8), 0, s>>>(c, sw, att, nstars, g0, li))
+    if (pairs && fuv_bricks(fnr, fnu)) NB_FUV_APPLY(FUV_BRICKS);
+    else if (pairs) NB_FUV_APPLY(FUV_PAIRS);
+    else NB_FUV_APPLY(FUV_PLAIN);
+#undef NB_FUV_APPLY
     return cudaGetLastError();
 }
