@@ -16,11 +16,11 @@
 //   y and z faces of plane p-1 (its slot is complete since the barrier), kept in registers but for
 //   the face above each row pair, which the next warp reads a step later from shared memory.
 // The faces at the tile's lower y and z edges and the state beyond its upper z edge are extra work
-// of two warps, done a step ahead.  128 registers, 108 KB of shared memory, two blocks per SM.
+// of two warps, done a step ahead.  128 registers, 112 KB of shared memory, two blocks per SM.
 //
 // Bound: instruction issue at 16 warps a SM (issue active ~60%; barrier, shared-memory and fixed
 // latencies about equal), not bytes and not one pipe: 320 / 340 thread instructions a cell where pairs
-// of components took 528 / 559.  Measured at 256^3 (sheet, 20-plane chunks): stage 1 309 -> 252 us,
+// of components took 528 / 559.  Measured at 256^3 (sheet, 20-plane chunks; 242 and 261 with the chosen depth): stage 1 309 -> 252 us,
 // stage 2 338 -> 271 us (2.40 and 3.22 TB/s of their 36 and 52 B a cell); 192^3 145 -> 121, 160 -> 130 us.
 // Tried on this tile and slower or level: the own cells' values read again from global memory (one
 // address instruction and a pointer load per access, +12%), shuffles along k (+3%), the march unrolled
@@ -36,7 +36,7 @@ constexpr int HYDRO_TJ = 16;          // tile rows along j (two rows per warp)
 constexpr int HYDRO_THREADS = 256;    // eight warps
 constexpr int PPW = 36;               // pairs per row of a plane: columns k0-2 .. k0+33
 constexpr long long HYDRO_IDX32_CELLS = (1LL << 31) - 1;       // signed cell offsets
-constexpr int HYDRO_MINB = 2;         // resident blocks per SM (128 registers, 80 KB of shared memory each)
+constexpr int HYDRO_MINB = 2;         // resident blocks per SM (128 registers, 112 KB of shared memory each)
 constexpr float HYDRO_PLANE[HYDRO_MINB + 1] = {0.0f, 0.74f, 1.0f};   // a plane's time by blocks on an SM
 constexpr int HYDRO_ROT_STEP = 2;     // two resident blocks place their extra work two schedulers apart
 
