@@ -293,7 +293,9 @@ typedef struct nb_pack_params {
  * handle's fields, the shock proxy computed inline when shock_on != 0, into `out8` (device,
  * 8 B/cell, C order [i][j][k][4] float16).  With smooth != 0 also render.py:281-298 smooth_axis
  * along x, y, z, with `tmp8` (device, 8 B/cell) as the second grid; the result is in out8
- * either way.  Renderer.pack packs into Sim.render_scratch (sim.py:821-825): the stage block. */
+ * either way.  Renderer.pack packs into Sim.render_scratch (sim.py:821-825): the stage block, whose
+ * planes 0-1 an ionization or a FUV pass uses too, plane 2 a FUV pass with the plane source, and all
+ * four a step. */
 int nb_render_pack(nb_handle h, const nb_pack_params* pp, int shock_on, int smooth, void* out8, void* tmp8);
 
 /* ---------------------------------------------------------------- diagnostics */

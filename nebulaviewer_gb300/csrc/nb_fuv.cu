@@ -7,12 +7,9 @@
 // inclusive group scan over a Kahan-compensated carry; a lane that crosses into new radial
 // bins writes them, and a ray stops once its optical depth passes 120 (exp(-tau) is 0.0f from
 // there on: its remaining bins are written as 0).  Density and ionized fraction are sampled at the
-// same corners, so each cell is first packed with its upper neighbour along k, (rho, xi) of both, into
-// free scratch (the four stage planes): four 16-byte gathers a sample instead of eight of 8 bytes, 126
-// instead of 159 million L1 wavefronts at 256^3, for twice the pack's bytes.  With its pack the cast
-// takes 570 instead of 590 us there, 182 for 201 at 128^3, 2066 for 2217 at 384^3; it is bound by the
-// chain of a segment (loads, scan, ballots: 57% of the issue slots) and L1 (76%).  All rays of all
-// active stars are one launch, into one attenuation table per star.  An entry is the pair (att(r), att(min(r + 1, nr - 1))) as one float2 (the ray writes each bin into
+// same corners, so they are first packed as (rho, xi) pairs into free scratch: one 8-byte gather per
+// corner.  All rays of all active stars are one launch, into one attenuation table per star.  An
+// entry is the pair (att(r), att(min(r + 1, nr - 1))) as one float2 (the ray writes each bin into
 // its own pair and its lower neighbour's), so a trilinear sample of apply_fuv is four 8-byte gathers
 // instead of eight 4-byte ones; values and arithmetic are those of the plain table
 // (NB_TUNE_FUV_PAIRS = 0), bit for bit, in whichever order the entries lie.  apply_fuv accumulates
@@ -23,24 +20,17 @@
 // table lies in bricks of 4 u x 4 r, one line each (a ray still writes whole 32-byte sectors), the
 // rays of a brick are cast together, and a warp of the apply takes 4 x 2 x 4 cells instead of 32
 // along k: 21 lines per cell group and star instead of 48.  apply_fuv at 64^3 / 192^3 / 256^3 /
-// 384^3 with six stars: 30 / 256 / 563 / 1954 -> 20 / 177 / 395 / 1298 us (cells alone 458 at
-// 256^3), now issue bound (88%); cast_fuv 630 -> 590 us at 256^3 (whole pairs where a ray fills its
-// last bins), level below 128^3.
+// 384^3 with six stars: 30 / 256 / 563 / 1954 -> 18 / 177 / 395 / 1298 us (cells alone 458 at
+// 256^3), now issue bound (88%); cast_fuv with its pack 630 -> 590 us at 256^3 (whole pairs where
+// a ray fills its last bins), level below 128^3.
 #include "nb_rayutil.cuh"
 
 namespace {
 
-// (rho, xi) of a cell and of its upper neighbour along k (its own in the last cell of a row)
 __global__ void __launch_bounds__(256) pack_rx_kernel(const float* __restrict__ rho, const float* __restrict__ xi,
-                                                      float4* __restrict__ rx, int nrow, int nz) {
-    for (int r = blockIdx.x * blockDim.y + threadIdx.y; r < nrow; r += gridDim.x * blockDim.y) {
-        const long long base = (long long)r * nz;
-        const float *rr = rho + base, *xr = xi + base;
-        for (int k = threadIdx.x; k < nz; k += 32) {
-            const int n = min(k + 1, nz - 1);
-            rx[base + k] = make_float4(rr[k], xr[k], rr[n], xr[n]);
-        }
-    }
+                                                      float2* __restrict__ rx, long long n) {
+    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x)
+        rx[q] = make_float2(rho[q], xi[q]);
 }
 
 // Layouts of an instance's attenuation table, per star.
@@ -67,7 +57,7 @@ __device__ __forceinline__ int fuv_r(int ir) {
 template <int G, int L>
 __global__ void __launch_bounds__(256, 5) cast_fuv_kernel(const NbConst* __restrict__ c, const NbStarW* __restrict__ sw,
                                                        const float4* __restrict__ dirs,
-                                                       const float4* __restrict__ rx,
+                                                       const float2* __restrict__ rx,
                                                        float* __restrict__ att, int nstars,
                                                        const float* star_override, float tau_cut) {
     const int nr = c->fnr, nu = c->fnu, nphi = c->fnphi, nray = nu * nphi;
@@ -324,11 +314,13 @@ static bool fuv_bricks(int fnr, int fnu) { return fnr % 4 == 0 && fnu % 4 == 0; 
 
 cudaError_t nb_launch_cast_fuv(const NbConst* c, const NbStarW* sw, const float4* dirs, const float* rho,
                                const float* xi, float* att, int nstars, int group, const float* star_override,
-                               int ref_layout, cudaStream_t s, int fnu, int fnphi, void* rx_scratch, long long ncell, int nz,
+                               int ref_layout, cudaStream_t s, int fnu, int fnphi, void* rx_scratch, long long ncell,
                                float tau_cut, int pairs, int fnr) {
-    float4* rx = static_cast<float4*>(rx_scratch);
-    const int nrow = (int)(ncell / nz);
-    pack_rx_kernel<<<nrow < 8 * 152 * 8 ? (nrow + 7) / 8 : 152 * 8, dim3(32, 8), 0, s>>>(rho, xi, rx, nrow, nz);
+    float2* rx = static_cast<float2*>(rx_scratch);
+    {
+        const long long b = (ncell + 255) / 256;
+        pack_rx_kernel<<<(int)(b < 152LL * 16 ? (b < 1 ? 1 : b) : 152LL * 16), 256, 0, s>>>(rho, xi, rx, ncell);
+    }
     const long long threads = (long long)fnu * fnphi * nstars * group;
     const int blocks = (int)((threads + 255) / 256);
 #define NB_FUV_LAUNCH(G, L) \

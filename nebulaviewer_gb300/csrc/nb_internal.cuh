@@ -300,10 +300,10 @@ cudaError_t nb_launch_ionize_batch(const NbRayJob* jobs, const NbRayJob* host_jo
 cudaError_t nb_launch_plane_front(const NbConst* c, const float* rho, float* xf, int ny, int nz, cudaStream_t s);
 cudaError_t nb_launch_plane_fuv(const NbConst* c, const float* rho, const float* xi, float* g, int ny, int nz,
                                 cudaStream_t s);
-// packs (rho, xi) of each cell and its upper neighbour into rx_scratch (ncell float4) first
+// packs (rho, xi) pairs into rx_scratch (ncell float2, 8-byte aligned) first
 cudaError_t nb_launch_cast_fuv(const NbConst* c, const NbStarW* sw, const float4* dirs, const float* rho,
                                const float* xi, float* att, int nstars, int group, const float* star_override,
-                               int ref_layout, cudaStream_t s, int fnu, int fnphi, void* rx_scratch, long long ncell, int nz,
+                               int ref_layout, cudaStream_t s, int fnu, int fnphi, void* rx_scratch, long long ncell,
                                float tau_cut, int pairs, int fnr);
 #define NB_FUV_TAU_CUT 120.0f            // optical depth past which a FUV ray's remaining bins are 0
 cudaError_t nb_launch_apply_fuv(const NbConst* c, const NbStarW* sw, const float* att, int nstars, void* g0,

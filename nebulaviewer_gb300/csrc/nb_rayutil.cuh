@@ -44,10 +44,9 @@ __device__ __forceinline__ float rcp_approx(float x) {
     return r;
 }
 
-// sample_n of two fields stored interleaved, each cell with its upper neighbour along k: entry k of a row
-// is ((rho, xi)(k), (rho, xi)(min(k + 1, nz - 1))).  The same corners, weights and float operations per
-// field as two sample_n calls, with four 16-byte loads.
-__device__ __forceinline__ float2 sample_n2(const float4* __restrict__ a, int nx, int ny, int nz, float px, float py,
+// sample_n of two fields stored interleaved ((rho, xi) pairs): the same corners, weights and
+// float operations per field as two sample_n calls, with one 8-byte load per corner.
+__device__ __forceinline__ float2 sample_n2(const float2* __restrict__ a, int nx, int ny, int nz, float px, float py,
                                            float pz, float dx, float inv_dx, bool pow2) {
     const float gx = (pow2 ? px * inv_dx : px / dx) - 0.5f;
     const float gy = (pow2 ? py * inv_dx : py / dx) - 0.5f;
@@ -58,21 +57,20 @@ __device__ __forceinline__ float2 sample_n2(const float4* __restrict__ a, int nx
     const float fx = gx - (float)i0, fy = gy - (float)j0, fz = gz - (float)k0;
     const int ia = iclampd(i0, 0, nx - 1), ib = iclampd(i0 + 1, 0, nx - 1);
     const int ja = iclampd(j0, 0, ny - 1), jb = iclampd(j0 + 1, 0, ny - 1);
-    const int ka = iclampd(k0, 0, nz - 1);
+    const int ka = iclampd(k0, 0, nz - 1), kb = iclampd(k0 + 1, 0, nz - 1);
     // as sample_n, always in the clamped form (an all-inside fast path measured slower in the FUV rays)
-    const float4* p = a + (((long long)ia * ny + ja) * nz + ka);
-    const int dj = (jb - ja) * nz, di = (ib - ia) * (ny * nz);
-    float4 q00 = __ldg(p), q10 = __ldg(p + di), q01 = __ldg(p + dj), q11 = __ldg(p + (di + dj));
-    if (k0 < 0) {                                       // below the first centre both corners are cell 0
-        q00.z = q00.x; q10.z = q10.x; q01.z = q01.x; q11.z = q11.x;
-        q00.w = q00.y; q10.w = q10.y; q01.w = q01.y; q11.w = q11.y;
-    }
+    const float2* p = a + (((long long)ia * ny + ja) * nz + ka);
+    const int dk = kb - ka, dj = (jb - ja) * nz, di = (ib - ia) * (ny * nz);
+    const float2 c000 = __ldg(p), c100 = __ldg(p + di);
+    const float2 c010 = __ldg(p + dj), c110 = __ldg(p + (di + dj));
+    const float2 c001 = __ldg(p + dk), c101 = __ldg(p + (di + dk));
+    const float2 c011 = __ldg(p + (dj + dk)), c111 = __ldg(p + (di + dj + dk));
     float out[2];
 #pragma unroll
     for (int f = 0; f < 2; ++f) {
-        const float v000 = f ? q00.y : q00.x, v100 = f ? q10.y : q10.x, v010 = f ? q01.y : q01.x;
-        const float v110 = f ? q11.y : q11.x, v001 = f ? q00.w : q00.z, v101 = f ? q10.w : q10.z;
-        const float v011 = f ? q01.w : q01.z, v111 = f ? q11.w : q11.z;
+        const float v000 = f ? c000.y : c000.x, v100 = f ? c100.y : c100.x, v010 = f ? c010.y : c010.x;
+        const float v110 = f ? c110.y : c110.x, v001 = f ? c001.y : c001.x, v101 = f ? c101.y : c101.x;
+        const float v011 = f ? c011.y : c011.x, v111 = f ? c111.y : c111.x;
         const float c00 = v000 + (v100 - v000) * fx;
         const float c10 = v010 + (v110 - v010) * fx;
         const float c01 = v001 + (v101 - v001) * fx;

@@ -484,7 +484,8 @@ class Sim:
     xi_tmp = property(lambda self: Field(self._stage[0]))
 
     def render_scratch(self):
-        """two RGBA16F grids (half4 views of the stage block), free between steps (sim.py:821-825)"""
+        """two RGBA16F grids (half4 views of the stage block), free between steps (sim.py:821-825):
+        planes 0-1 and planes 2-3"""
         b = self._stage.view(torch.float16).reshape(-1)
         n = self._n
         return (Field(b[:4 * n].view(self.shape + (4,))), Field(b[4 * n:8 * n].view(self.shape + (4,))))
@@ -928,7 +929,9 @@ class Sim:
         """render.py:176-205 pack_volume_lm (+ render.py:281-298 smooth_axis x, y, z): the RGBA16F
         voxel grid (emission r, g, b; dust) of the current fields, packed into the render scratch
         (the stage block, free between steps) as Renderer.pack does; returns it as a
-        (nx, ny, nz, 4) float16 Field.  `pp`: the reference's PackParams (render.py:77-88,
+        (nx, ny, nz, 4) float16 Field, a view: the smoothed voxels (planes 2-3) hold until the next
+        step, voxel pack or, with a plane source, FUV pass; those of smooth=False (planes 0-1) until
+        the next ionization or FUV pass too.  `pp`: the reference's PackParams (render.py:77-88,
         Renderer.pack_params) or a mapping with the same keys; shock_on defaults to any(c_sh)."""
         get = (lambda k: pp[k]) if isinstance(pp, dict) else (lambda k: getattr(pp, k))
         vals = {k: get(k) for k in self.PACK_FIELDS}
