@@ -16,7 +16,8 @@
 //   y and z faces of plane p-1 (its slot is complete since the barrier), kept in registers but for
 //   the face above each row pair, which the next warp reads a step later from shared memory.
 // The faces at the tile's lower y and z edges and the state beyond its upper z edge are extra work
-// of two warps, done a step ahead.  128 registers, 112 KB of shared memory, two blocks per SM.
+// of two warps, done a step ahead.  128 registers, 112 KB of shared memory, two blocks per SM at any
+// number of stars.
 //
 // Bound: instruction issue at 16 warps a SM (issue active ~60%; barrier, shared-memory and fixed
 // latencies about equal), not bytes and not one pipe: 320 / 340 thread instructions a cell where pairs
@@ -193,10 +194,14 @@ struct HydroSmem {
     static constexpr int BAR_BYTES = 64;
     static constexpr int FIXED = PRIM + 3 * SLOT + BAR_BYTES;
     static constexpr int FLAG = FIXED - BAR_BYTES + 16;                      // after two mbarriers: a wait gave up
-    // star tables: positions / wind weights and jets (2 x float4 per star), then the tile's jet
-    // list: a count and the indices (one byte each) of the stars whose jet can reach the tile
-    __host__ __device__ static int jet_list_offset(int nstars) { return FIXED + nstars * 32; }
-    static int bytes(int nstars) { return jet_list_offset(nstars) + 16 + ((nstars + 15) & ~15); }
+    // The tile's jet list: a count and the indices (one byte each) of the stars whose jet can reach the tile.
+    // The stars' weights and jets are read through L1, by all lanes at once: two blocks leave 1.3 KB of an
+    // SM's shared memory, and with the tables there (32 B a star) from 38 stars on only one block was resident.
+    // Stages 1 + 2 at 256^3 with the tables there -> this, in 37-plane chunks: 6 stars 512 -> 514 us, 40 stars
+    // 846 -> 618, 128 stars 1343 -> 1135, 256 stars 2369 -> 2074; without winds from 38 stars on 662 -> 491.
+    static constexpr int JETS = FIXED;
+    static int bytes(int nstars) { return JETS + 16 + ((nstars + 15) & ~15); }
+    static_assert(HYDRO_MINB * (JETS + 16 + NB_MAX_STARS + 1024) <= 228 * 1024, "two blocks per SM");
 };
 
 // One (j,k) tile column of one instance, marched over its i-chunk.  Called once per block by
@@ -221,10 +226,8 @@ __device__ __forceinline__ void hydro_tile(const HydroLaunch& L, int tile, unsig
         smem += zero;
     }
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + SM::FIXED - SM::BAR_BYTES);
-    float4* sw_w = reinterpret_cast<float4*>(smem + SM::FIXED);
     const NbConst& C = *L.c;
     const int nx = C.nx, ny = C.ny, nz = C.nz, nstars = L.no_sources ? 0 : C.nstars;
-    float4* sw_j = sw_w + nstars;
 
     const int tid = threadIdx.x, tk = tid & 31, tj = tid >> 5;
     const HydroTile tl(L, tile, nx, TJ);
@@ -236,12 +239,8 @@ __device__ __forceinline__ void hydro_tile(const HydroLaunch& L, int tile, unsig
     const float pulse = L.use_override ? L.pulse_override : L.st->pulse_f;
     const float wind = L.no_sources ? 0.0f : C.wind_f, jet_cos = C.jet_cos_f, jet_r = C.jet_r_f;
 
-    int* n_jet_p = reinterpret_cast<int*>(smem + SM::jet_list_offset(nstars));
-    unsigned char* jet_ix = smem + SM::jet_list_offset(nstars) + 16;
-    for (int s = tid; s < nstars; s += blockDim.x) {
-        sw_w[s] = L.sw[s].w;
-        sw_j[s] = L.sw[s].jet;
-    }
+    int* n_jet_p = reinterpret_cast<int*>(smem + SM::JETS);
+    unsigned char* jet_ix = smem + SM::JETS + 16;
     auto issue = [&](int p, int to, uint64_t* b) {           // plane p into the raw slot at `to`, tracked by b
         if (!L.maps) return;                     // failure-path test: the wait for it runs out
         const int pc = iclampd(p, 0, nx - 1);
@@ -334,20 +333,21 @@ __device__ __forceinline__ void hydro_tile(const HydroLaunch& L, int tile, unsig
             const float px = ((float)i + 0.5f) * dx, py0 = ((float)j + 0.5f) * dx, py1 = ((float)(j + 1) + 0.5f) * dx;
             const float pz = ((float)k + 0.5f) * dx;
             if (wind > 0.0f && (x.x > 0.01f || x.y > 0.01f)) {
+                // an inactive star adds exactly nothing (a zero weight at the origin: no branch, so that
+                // four stars' loads and reciprocals are under way together)
                 F2 ax = vset<F2>(0.0f), ay = ax, az = ax;
+#pragma unroll 4
                 for (int s = 0; s < nstars; ++s) {
-                    const float4 st = sw_w[s];
-                    if (st.w > 0.0f) {
-                        const float rx = px - st.x, rz = pz - st.z;
-                        const F2 ry = mk2(py0 - st.y, py1 - st.y);
-                        const F2 r2 = vadd(vfma(ry, ry, vset<F2>(rx * rx + rz * rz)), vset<F2>(0.0004f));
-                        const F2 f = vmul(vset<F2>(st.w), vrcp(vmul(r2, mk2(sqrtf(lo(r2)), sqrtf(hi(r2))))));
-                        ax = vfma(vset<F2>(rx), f, ax);
-                        ay = vfma(ry, f, ay);
-                        az = vfma(vset<F2>(rz), f, az);
-                    }
+                    float4 st = __ldg(&L.sw[s].w);
+                    if (!(st.w > 0.0f)) st = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    const float rx = px - st.x, rz = pz - st.z;
+                    const F2 ry = mk2(py0 - st.y, py1 - st.y);
+                    const F2 r2 = vadd(vfma(ry, ry, vset<F2>(rx * rx + rz * rz)), vset<F2>(0.0004f));
+                    const F2 f = vmul(vset<F2>(st.w), vrcp(vmul(r2, mk2(sqrtf(lo(r2)), sqrtf(hi(r2))))));
+                    ax = vfma(vset<F2>(rx), f, ax);
+                    ay = vfma(ry, f, ay);
+                    az = vfma(vset<F2>(rz), f, az);
                 }
-                // cells at or below an ionized fraction of 0.01 take no wind
                 // cells at or below an ionized fraction of 0.01 take no wind
                 const F2 wx = vmul(rho, mk2(x.x > 0.01f ? wind * x.x : 0.0f, x.y > 0.01f ? wind * x.y : 0.0f));
                 S.n = vfma(wx, ax, S.n);
@@ -358,7 +358,7 @@ __device__ __forceinline__ void hydro_tile(const HydroLaunch& L, int tile, unsig
                 float jx[2] = {0.0f, 0.0f}, jy[2] = {0.0f, 0.0f}, jz[2] = {0.0f, 0.0f};
                 for (int m = 0; m < n_jet; ++m) {
                     const int s = jet_ix[m];
-                    const float4 jt = sw_j[s], st = sw_w[s];
+                    const float4 jt = __ldg(&L.sw[s].jet), st = __ldg(&L.sw[s].w);
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
                         const float rx = px - st.x, ry = (h ? py1 : py0) - st.y, rz = pz - st.z;
