@@ -37,7 +37,8 @@ struct nb_instance {
     int nstars = 0, star_alloc = 0;
     long long host_it = 0;
     int smax_valid = 0;
-    int chunk_i = 20, chunk_set = 0;    // planes per hydro tile, chosen for the grid (nb_create) or set (nb_set_tuning)
+    int chunk_i = 0, chunk_set = 0;     // planes per hydro tile as set (nb_set_tuning)
+    int depth[2] = {20, 20};            // ... else as chosen for the grid: without winds, with the stars' (chosen_depth)
     int ray_group = 1, fuv_group = 16;  // measured best at 192^3-256^3 (nb_set_tuning)
     int tile_order = 0;
     int front_cull = 1;                 // apply_front skips the stars that cannot change a segment
@@ -164,6 +165,10 @@ long long hydro_columns(const nb_desc& d) {
     return (long long)((d.nz + 31) / 32) * ((d.ny + tj - 1) / tj);
 }
 
+// planes per hydro tile of the single-instance stages (no_sources: a stirring-phase stage)
+int chosen_depth(const nb_instance* h, bool no_sources) { return h->depth[!no_sources && h->hc.wind_f > 0.0f]; }
+int chunk_depth(const nb_instance* h, bool no_sources) { return h->chunk_set ? h->chunk_i : chosen_depth(h, no_sources); }
+
 float* plane(nb_instance* h, int p) { return h->d.f.stage + (long long)p * h->ncell; }
 
 int launch_stage(nb_instance* h, const float* const in[4], const float* const u0[4], float* const out[4], int map_in,
@@ -191,7 +196,7 @@ int launch_stage(nb_instance* h, const float* const in[4], const float* const u0
     const int tj = nb_hydro_tile_j();
     L.tiles_k = (h->d.nz + 31) / 32;
     L.tiles_j = (h->d.ny + tj - 1) / tj;
-    L.chunk_i = h->chunk_i < h->d.nx ? h->chunk_i : h->d.nx;
+    L.chunk_i = std::min(chunk_depth(h, no_sources), h->d.nx);
     L.n_chunks = (h->d.nx + L.chunk_i - 1) / L.chunk_i;
     L.nstars_host = h->nstars;
     L.order = h->tile_order;
@@ -343,7 +348,7 @@ NB_EXPORT int nb_create(const nb_desc* d, nb_handle* out) {
         delete h;
         return fail(nullptr, NB_ERR_LIMIT, "grid too large (ny * nz and fnu * fnphi * fnr must stay below 2^31)");
     }
-    h->chunk_i = nb_hydro_depth(d->nx, hydro_columns(*d), sm_count());
+    h->depth[0] = h->depth[1] = nb_hydro_depth(d->nx, hydro_columns(*d), sm_count(), 0);
     NbConst& c = h->hc;
     c.nx = d->nx; c.ny = d->ny; c.nz = d->nz; c.nstars = 0;
     c.dx_pow2 = is_pow2(d->dx) ? 1 : 0;
@@ -519,6 +524,7 @@ NB_EXPORT int nb_set_stars(nb_handle h, const nb_star* s, int n) {
         tmp[i].kind = s[i].kind; tmp[i].jkind = s[i].jkind;
     }
     if (n > 0) CK(h, cudaMemcpyAsync(h->stars, tmp, sizeof(NbStarDev) * n, cudaMemcpyHostToDevice, h->stream));
+    if (n != h->nstars) h->depth[1] = nb_hydro_depth(h->d.nx, hydro_columns(h->d), sm_count(), n);
     h->nstars = n;
     h->hc.nstars = n;
     return upload_const(h);
@@ -910,7 +916,7 @@ NB_EXPORT int nb_shock(nb_handle h, float* out) {
 NB_EXPORT int nb_get_tuning(nb_handle h, int key, int* value) {
     if (!h || !value) return fail(h, NB_ERR_ARG, "null argument");
     switch (key) {
-        case NB_TUNE_CHUNK_I: *value = h->chunk_i; return NB_OK;
+        case NB_TUNE_CHUNK_I: *value = chunk_depth(h, false); return NB_OK;
         case NB_TUNE_RAY_GROUP: *value = h->ray_group; return NB_OK;
         case NB_TUNE_FUV_GROUP: *value = h->fuv_group; return NB_OK;
         case NB_TUNE_TILE_ORDER: *value = h->tile_order; return NB_OK;
@@ -1199,8 +1205,12 @@ NB_EXPORT int nb_batch_create(const nb_handle* hs, const int* ion_every, int n, 
     b->active.assign(n, 1);
     b->n_active = n;
     double planes = 0.0;
-    for (auto* h : b->inst) planes += (double)hydro_columns(h->d) * h->d.nx;
-    const int depth = nb_hydro_depth_batch(planes, b->grid);
+    int winds = 0;
+    for (auto* h : b->inst) {
+        planes += (double)hydro_columns(h->d) * h->d.nx;
+        if (h->hc.wind_f > 0.0f) winds = std::max(winds, h->nstars);
+    }
+    const int depth = nb_hydro_depth_batch(planes, b->grid, winds);
     for (int i = 0; i < n; ++i) {
         nb_instance* h = b->inst[i];
         bi[i] = NbBatchInst{h->c, h->st, h->stars, h->sw, h->nstars, 1, h->front_bounds};

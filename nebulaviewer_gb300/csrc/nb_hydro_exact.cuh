@@ -19,6 +19,7 @@ constexpr int HYDRO_TJ = 8;           // tile rows along j (one warp per row; 16
 constexpr long long HYDRO_IDX32_CELLS = (1LL << 31) - 1;       // signed cell offsets
 constexpr int HYDRO_MINB = 4;         // resident blocks per SM the register budget is sized for (64 regs)
 constexpr float HYDRO_PLANE[HYDRO_MINB + 1] = {0.0f, 0.59f, 0.72f, 0.86f, 1.0f};   // a plane's time by blocks on an SM
+constexpr double HYDRO_WIND = 0.04;   // one star's wind over an ionized plane of a tile, in planes (nb_hydro_depth)
 constexpr int HYDRO_ROT_STEP = 1;     // resident blocks start their extra work one scheduler apart
 
 __device__ __forceinline__ float comp(const float4& v, int c) {

@@ -39,6 +39,7 @@ constexpr int PPW = 36;               // pairs per row of a plane: columns k0-2 
 constexpr long long HYDRO_IDX32_CELLS = (1LL << 31) - 1;       // signed cell offsets
 constexpr int HYDRO_MINB = 2;         // resident blocks per SM (128 registers, 112 KB of shared memory each)
 constexpr float HYDRO_PLANE[HYDRO_MINB + 1] = {0.0f, 0.74f, 1.0f};   // a plane's time by blocks on an SM
+constexpr double HYDRO_WIND = 0.04;   // one star's wind over an ionized plane of a tile, in planes (nb_hydro_depth)
 constexpr int HYDRO_ROT_STEP = 2;     // two resident blocks place their extra work two schedulers apart
 
 // an approximate reciprocal (<= 1 ulp)

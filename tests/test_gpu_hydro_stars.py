@@ -88,3 +88,19 @@ def test_idle_stars_do_not_slow_the_stage():
         t[nstars] = stage_ms(s)
         s.close()
     assert t[256] <= 1.15 * t[1], t
+
+
+def test_chosen_depth_with_many_winds():
+    """the depth chosen for a grid counts its stars' winds: many winds make the ionized tiles the slow ones,
+    and few deep chunks then leave the GPU waiting for them.  The chosen depth is within a quarter of the
+    better of two fixed ones (one for the whole column was three times as slow)."""
+    from nebulaviewer_gb300 import autotune as at
+    for res, nstars in ((192, 256), (384, 64)):
+        s = sheet(res, nstars, 0.5)
+        s.step(12)
+        chosen, t = stage_ms(s), {}
+        for depth in (8, 24):
+            at.put(s, "chunk_i", depth)
+            t[depth] = stage_ms(s)
+        assert chosen <= 1.25 * min(t.values()), (res, nstars, chosen, t)
+        s.close()
