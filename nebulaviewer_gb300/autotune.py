@@ -32,7 +32,7 @@ _CACHE = {}
 
 def _key(sim):
     return (tuple(sim.shape), len(sim.stars), tuple(sim.rfront.shape), tuple(sim.att.shape), sim.P.get("solver"),
-            sim.arith)
+            sim.P.get("limiter"), float(sim.P.get("wind", 0.0)) > 0.0, sim.arith)
 
 
 def get(sim, knob):
@@ -93,7 +93,8 @@ def autotune(sim, knobs=None, steps=4, use_cache=True):
     try:
         for knob in knobs:
             best = None
-            # the library's own choice of the depth competes with the fixed ones
+            # the library's own choice of the depth competes with the fixed ones (putting it back leaves the
+            # choice to the library)
             extra = (orig[knob],) if knob == "chunk_i" and orig[knob] not in CANDIDATES[knob] else ()
             for v in CANDIDATES[knob] + extra:
                 put(sim, knob, v)

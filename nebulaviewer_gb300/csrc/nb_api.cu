@@ -935,8 +935,10 @@ NB_EXPORT int nb_set_tuning(nb_handle h, int key, int value) {
     switch (key) {
         case NB_TUNE_CHUNK_I:
             if (value < 1) return fail(h, NB_ERR_ARG, "chunk_i must be >= 1");
+            // the chosen depth itself leaves the choice to the library: a tuner that puts back what it read,
+            // or prefers the library's depth, must not pin it for other stars or for a batch
             h->chunk_i = value;
-            h->chunk_set = 1;
+            h->chunk_set = value != chosen_depth(h, false);
             return NB_OK;
         case NB_TUNE_TILE_ORDER:
             if (value != 0 && value != 1) return fail(h, NB_ERR_ARG, "tile order must be 0 or 1");
