@@ -25,6 +25,7 @@
 #include <cstring>
 
 #include "nb_f32x2.cuh"
+#include "nb_rays_rule.h"
 #include "nb_rayutil.cuh"
 
 namespace {
@@ -168,8 +169,8 @@ __device__ __noinline__ int2 ray_range(const NbConst& C, float sx, float sy, flo
 // cast_ray with one lane per ray, as a plain loop, where nb_rays_small allows it: the same bits (the
 // products and sums are spelled out where a contraction would change them).  Along the part of the ray
 // that lies a cell inside the box, [i0, i1], the eight corners lie at fixed steps from the lower one, and
-// neither a clamp nor a test of the domain is needed; the half cell to spare is far above the rounding of
-// i0 and i1, which may be approximate.  floor(g) is g added to 1.5 x 2^23 rounded down, whose bits also
+// neither a clamp nor a test of the domain is needed; nb_rays_small keeps the rounding of i0 and i1, which
+// may be approximate, and of the positions below the half cell to spare.  floor(g) is g added to 1.5 x 2^23 rounded down, whose bits also
 // hold the index: no conversion instruction (those issue at an eighth of the rate).  Samples before i0 and
 // after i1 are sample_n's.  A star inside that part starts at sample 0, so a ray that ends within it never
 // needs its exact range, which costs eight divisions.
@@ -756,14 +757,7 @@ cudaError_t nb_launch_ray_order(int nu, int nphi, const float4* dirs, float4* ou
     return cudaGetLastError();
 }
 
-// cast_ray1's rule, on the host: cells, samples and the index of a corner are exact in its floats and
-// 32-bit integers, the part of the box a cell from its faces is there, and the cell size keeps every
-// product and quotient of positions normal.
-int nb_rays_small(const NbConst& c) {
-    const int most = 1 << 16;
-    return c.nx >= 4 && c.ny >= 4 && c.nz >= 4 && c.nx <= most && c.ny <= most && c.nz <= most &&
-           (long long)c.nx * c.ny * c.nz < (1LL << 31) && c.nsteps <= (1 << 22) && c.dx > 1e-12f && c.dx < 1e12f;
-}
+int nb_rays_small(const NbConst& c) { return nb_march_unclamped(c.nx, c.ny, c.nz, c.nsteps, c.dr_f, c.dx) ? 1 : 0; }
 
 cudaError_t nb_launch_cast_rays(const NbConst* c, const NbStarW* sw, const float4* dirs, const float* rho,
                                 float* rfront, int nstars, int group, uint2* bounds, const float* star_override,
