@@ -1207,14 +1207,10 @@ NB_EXPORT int nb_batch_create(const nb_handle* hs, const int* ion_every, int n, 
     b->active.assign(n, 1);
     b->n_active = n;
     double planes = 0.0;
-    int winds = 0;
-    for (auto* h : b->inst) {
-        planes += (double)hydro_columns(h->d) * h->d.nx;
-        if (h->hc.wind_f > 0.0f) winds = std::max(winds, h->nstars);
-    }
-    const int depth = nb_hydro_depth_batch(planes, b->grid, winds);
+    for (auto* h : b->inst) planes += (double)hydro_columns(h->d) * h->d.nx;
     for (int i = 0; i < n; ++i) {
         nb_instance* h = b->inst[i];
+        const int depth = nb_hydro_depth_batch(planes, b->grid, h->hc.wind_f > 0.0f ? h->nstars : 0);
         bi[i] = NbBatchInst{h->c, h->st, h->stars, h->sw, h->nstars, 1, h->front_bounds};
         L1[i] = stage_desc(h, false, depth);
         L2[i] = stage_desc(h, true, depth);

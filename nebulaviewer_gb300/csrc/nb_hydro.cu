@@ -327,7 +327,8 @@ int nb_hydro_depth(int nx, long long columns, int sms, int winds) {
 // The depth of a batch's stages, whose persistent blocks (`slots` of them) take tiles in turn: deep
 // chunks convert fewer halo planes (4.5 per chunk), shallow ones end together (half a chunk idle at the
 // end, and a chunk's wind work, as above); the sum is least at the depth whose square is 9 planes' worth
-// of each block's share, less by the winds.
+// of each block's share, less by the instance's own winds (a batch step of seven 128^3 with one star and a
+// 96^3 with 256 stars 2438 -> 1243 us; 1413 with the most windy instance's depth for all).
 int nb_hydro_depth_batch(double column_planes, int slots, int winds) {
     const double d = std::sqrt(9.0 * column_planes / (slots > 0 ? slots : 1) / (1.0 + 2.0 * HYDRO_WIND * winds));
     return d < 2.0 ? 2 : (d > 128.0 ? 128 : (int)d);
