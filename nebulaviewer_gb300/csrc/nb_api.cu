@@ -765,11 +765,13 @@ NB_EXPORT int nb_fuv(nb_handle h) {
         Prof pf(h, NB_PROF_CTRL, 1);
         CK(h, nb_launch_weights(h->c, h->st, h->stars, h->sw, h->nstars, nullptr, h->stream));
     }
+    const int layout = !h->fuv_pairs ? FUV_PLAIN
+                       : nb_fuv_bricks(h->d.fnr, h->d.fnu, h->d.fnphi, h->ncell) ? FUV_BRICKS : FUV_PAIRS;
     if (h->nstars > 0) {
         Prof pf(h, NB_PROF_CAST_FUV, 2);                // the (rho, xi) pack into stage planes 0-1 + the rays
         CK(h, nb_launch_cast_fuv(h->c, h->sw, h->dirs_fuv, h->d.f.rho, h->d.f.xi, h->att, h->nstars, h->fuv_group,
-                                 nullptr, 0, h->stream, h->d.fnu, h->d.fnphi, plane(h, 0), h->ncell,
-                                 h->fuv_cut ? NB_FUV_TAU_CUT : 0.0f, h->fuv_pairs, h->d.fnr));
+                                 nullptr, h->stream, h->d.fnu, h->d.fnphi, plane(h, 0), h->ncell,
+                                 h->fuv_cut ? NB_FUV_TAU_CUT : 0.0f, layout));
     }
     if (h->hc.plane_on) {
         Prof pf(h, NB_PROF_CAST_FUV, 1);
@@ -778,7 +780,7 @@ NB_EXPORT int nb_fuv(nb_handle h) {
     {
         Prof pf(h, NB_PROF_APPLY_FUV, 1);
         CK(h, nb_launch_apply_fuv(h->c, h->sw, h->att, h->nstars, h->d.f.g0, h->stream, h->d.nx,
-                                  h->d.ny, h->d.fields_fp32 ? 0 : 1, h->fuv_pairs, h->d.fnr, h->d.fnu));
+                                  h->d.ny, h->d.fields_fp32 ? 0 : 1, layout));
     }
     return NB_OK;
 }
@@ -827,9 +829,9 @@ NB_EXPORT int nb_cast_fuv(nb_handle h, const double xyz[3], float* att_out) {
     if (!h || !xyz || !att_out) return fail(h, NB_ERR_ARG, "null argument");
     float s3[4] = {(float)xyz[0], (float)xyz[1], (float)xyz[2], 0.f};
     CK(h, cudaMemcpyAsync(h->scratch3, s3, sizeof(s3), cudaMemcpyHostToDevice, h->stream));
-    CK(h, nb_launch_cast_fuv(h->c, h->sw, h->dirs_fuv, h->d.f.rho, h->d.f.xi, att_out, 1, 32, h->scratch3, 1,
+    CK(h, nb_launch_cast_fuv(h->c, h->sw, h->dirs_fuv, h->d.f.rho, h->d.f.xi, att_out, 1, 32, h->scratch3,
                              h->stream, h->d.fnu, h->d.fnphi, plane(h, 0), h->ncell, h->fuv_cut ? NB_FUV_TAU_CUT : 0.0f,
-                             0, h->d.fnr));
+                             FUV_REF));
     CK(h, cudaStreamSynchronize(h->stream));
     return NB_OK;
 }

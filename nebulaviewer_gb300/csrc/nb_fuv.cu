@@ -33,13 +33,6 @@ __global__ void __launch_bounds__(256) pack_rx_kernel(const float* __restrict__ 
         rx[q] = make_float2(rho[q], xi[q]);
 }
 
-// Layouts of an instance's attenuation table, per star.
-enum {
-    FUV_PLAIN,      // [u][phi][r], one float
-    FUV_PAIRS,      // [u][phi][r], (att(r), att(min(r + 1, nr - 1)))
-    FUV_BRICKS,     // the pairs, [phi][u / 4][r / 4][u % 4][r % 4]: a 128-byte line holds 4 u x 4 r
-    FUV_REF         // [r][u][phi], one float (a cast into the caller's array)
-};
 // An entry's offset is the sum of three: of its phi, its u and its r.
 template <int L>
 __device__ __forceinline__ int fuv_phi(int ip, int nu, int nr) {
@@ -186,15 +179,16 @@ __global__ void __launch_bounds__(256, 6) apply_fuv_kernel(const NbConst* __rest
     const float* C_plane_g0 = c->plane_g0;
     // a block takes 2^li x 2^lj rows, a warp 4 cells of each of them at a time
     const int lj = 3 - li, nbj = (ny + (1 << lj) - 1) >> lj, bi = blockIdx.x / nbj, bj = blockIdx.x - bi * nbj;
+    const int row = threadIdx.x >> 2;
     // per-row azimuth constants (star_row_table): the same values the per-cell form computes
     float4* tab = nullptr;
     if (nstars <= NB_ROW_STARS) {
         const int r = threadIdx.y, i = (bi << li) + (r >> lj), j = (bj << lj) + (r & ((1 << lj) - 1));
         star_row_table(st, act, nstars, ((float)i + 0.5f) * dx, ((float)j + 0.5f) * dx, nphi, colmul, rowtab[r]);
         __syncthreads();
-        tab = rowtab[threadIdx.x >> 2];
+        tab = rowtab[row];
     }
-    const int row = threadIdx.x >> 2, wi = (bi << li) + (row >> lj), wj = (bj << lj) + (row & ((1 << lj) - 1));
+    const int wi = (bi << li) + (row >> lj), wj = (bj << lj) + (row & ((1 << lj) - 1));
     if (wi >= nx || wj >= ny) return;
     const float px = ((float)wi + 0.5f) * dx, py = ((float)wj + 0.5f) * dx;
     const long long base = ((long long)wi * ny + wj) * nz;
@@ -308,14 +302,22 @@ cudaError_t nb_launch_plane_fuv(const NbConst* c, const float* rho, const float*
     return cudaGetLastError();
 }
 
-// Bricks where they need no padding: a table is then as large as in the other orders.  (Every ray
-// budget a simulation chooses for itself is a multiple of 4.)
-static bool fuv_bricks(int fnr, int fnu) { return fnr % 4 == 0 && fnu % 4 == 0; }
+// The layout of an instance's table where it holds pairs.  Bricks where they need no padding (a table is then
+// as large as in the other orders; every ray budget a simulation chooses for itself is a multiple of 4) and
+// where the cells that read it are many enough: a ray's bins then lie in four times as many lines, which costs
+// the cast what the table's size says, and the apply gains what the cells' number says.  Cast + apply of six
+// stars, bricks and [u][phi][r], at entries / cells of 1024 (16^3) 97 and 84 us, 16 (64^3) 156 and 156, 8
+// (80^3) 187 and 191, 5 (96^3) 213 and 228, 2 (128^3) 285 and 323; thin grids, three stars: 12 x 300 x 200 at
+// 11 119 and 113, 16 x 512 x 64 at 8 79 and 72, 512 x 512 x 4 at 4 136 and 138.  ([u][phi][r] with the cells
+// along k, before the bricks: 87 at 16^3, 164 at 64^3, 232 at 96^3, 85 at 16 x 512 x 64.)
+int nb_fuv_bricks(int fnr, int fnu, int fnphi, long long ncell) {
+    return fnr % 4 == 0 && fnu % 4 == 0 && (long long)fnr * fnu * fnphi <= 6 * ncell;
+}
 
 cudaError_t nb_launch_cast_fuv(const NbConst* c, const NbStarW* sw, const float4* dirs, const float* rho,
                                const float* xi, float* att, int nstars, int group, const float* star_override,
-                               int ref_layout, cudaStream_t s, int fnu, int fnphi, void* rx_scratch, long long ncell,
-                               float tau_cut, int pairs, int fnr) {
+                               cudaStream_t s, int fnu, int fnphi, void* rx_scratch, long long ncell,
+                               float tau_cut, int layout) {
     float2* rx = static_cast<float2*>(rx_scratch);
     {
         const long long b = (ncell + 255) / 256;
@@ -331,11 +333,11 @@ cudaError_t nb_launch_cast_fuv(const NbConst* c, const NbStarW* sw, const float4
         case 16: NB_FUV_LAUNCH(16, L); break;     \
         default: NB_FUV_LAUNCH(32, L); break;     \
     }
-    if (ref_layout) {
+    if (layout == FUV_REF) {
         NB_FUV_LAUNCH(32, FUV_REF);
-    } else if (pairs && fuv_bricks(fnr, fnu)) {
+    } else if (layout == FUV_BRICKS) {
         NB_FUV_GROUPS(FUV_BRICKS)
-    } else if (pairs) {
+    } else if (layout == FUV_PAIRS) {
         NB_FUV_GROUPS(FUV_PAIRS)
     } else {
         NB_FUV_GROUPS(FUV_PLAIN)
@@ -346,7 +348,7 @@ cudaError_t nb_launch_cast_fuv(const NbConst* c, const NbStarW* sw, const float4
 }
 
 cudaError_t nb_launch_apply_fuv(const NbConst* c, const NbStarW* sw, const float* att, int nstars, void* g0,
-                                cudaStream_t s, int nx, int ny, int half, int pairs, int fnr, int fnu) {
+                                cudaStream_t s, int nx, int ny, int half, int layout) {
     // 4 x 2 rows a block, or another split where that leaves far more lanes without a row (thin and small
     // grids): 2 x 4 and 1 x 8 rows took 10% longer at 192^3 and 256^3
     int li = 2, blocks = ((nx + 3) / 4) * ((ny + 1) / 2);
@@ -356,8 +358,8 @@ cudaError_t nb_launch_apply_fuv(const NbConst* c, const NbStarW* sw, const float
 #define NB_FUV_APPLY(L)                                                                                   \
     (half ? apply_fuv_kernel<true, L><<<blocks, dim3(32, 8), 0, s>>>(c, sw, att, nstars, g0, li)          \
           : apply_fuv_kernel<false, L><<<blocks, dim3(32, 8), 0, s>>>(c, sw, att, nstars, g0, li))
-    if (pairs && fuv_bricks(fnr, fnu)) NB_FUV_APPLY(FUV_BRICKS);
-    else if (pairs) NB_FUV_APPLY(FUV_PAIRS);
+    if (layout == FUV_BRICKS) NB_FUV_APPLY(FUV_BRICKS);
+    else if (layout == FUV_PAIRS) NB_FUV_APPLY(FUV_PAIRS);
     else NB_FUV_APPLY(FUV_PLAIN);
 #undef NB_FUV_APPLY
     return cudaGetLastError();

@@ -301,14 +301,22 @@ cudaError_t nb_launch_ionize_batch(const NbRayJob* jobs, const NbRayJob* host_jo
 cudaError_t nb_launch_plane_front(const NbConst* c, const float* rho, float* xf, int ny, int nz, cudaStream_t s);
 cudaError_t nb_launch_plane_fuv(const NbConst* c, const float* rho, const float* xi, float* g, int ny, int nz,
                                 cudaStream_t s);
-// packs (rho, xi) pairs into rx_scratch (ncell float2, 8-byte aligned) first
+// Layouts of an instance's attenuation table, per star.
+enum {
+    FUV_PLAIN,      // [u][phi][r], one float
+    FUV_PAIRS,      // [u][phi][r], (att(r), att(min(r + 1, nr - 1)))
+    FUV_BRICKS,     // the pairs, [phi][u / 4][r / 4][u % 4][r % 4]: a 128-byte line holds 4 u x 4 r
+    FUV_REF         // [r][u][phi], one float (a cast into the caller's array)
+};
+int nb_fuv_bricks(int fnr, int fnu, int fnphi, long long ncell);     // a table of pairs lies in bricks
+// packs (rho, xi) pairs into rx_scratch (ncell float2, 8-byte aligned) first; layout: of att
 cudaError_t nb_launch_cast_fuv(const NbConst* c, const NbStarW* sw, const float4* dirs, const float* rho,
                                const float* xi, float* att, int nstars, int group, const float* star_override,
-                               int ref_layout, cudaStream_t s, int fnu, int fnphi, void* rx_scratch, long long ncell,
-                               float tau_cut, int pairs, int fnr);
+                               cudaStream_t s, int fnu, int fnphi, void* rx_scratch, long long ncell,
+                               float tau_cut, int layout);
 #define NB_FUV_TAU_CUT 120.0f            // optical depth past which a FUV ray's remaining bins are 0
 cudaError_t nb_launch_apply_fuv(const NbConst* c, const NbStarW* sw, const float* att, int nstars, void* g0,
-                                cudaStream_t s, int nx, int ny, int half, int pairs, int fnr, int fnu);
+                                cudaStream_t s, int nx, int ny, int half, int layout);
 cudaError_t nb_launch_pack(const NbConst* c, const float* rho, const float* mx, const float* my, const float* mz,
                            const float* xi, const void* df, const void* g0, int half, void* out, long long n,
                            cudaStream_t s);
