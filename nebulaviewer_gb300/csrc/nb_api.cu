@@ -38,7 +38,8 @@ struct nb_instance {
     long long host_it = 0;
     int smax_valid = 0;
     int chunk_i = 0, chunk_set = 0;     // planes per hydro tile as set (nb_set_tuning)
-    int depth[2] = {20, 20};            // ... else as chosen for the grid: without winds, with the stars' (chosen_depth)
+    int depth[2] = {20, 20};            // ... else as chosen for the grid: without winds and jets, with the stars' (choose_depth)
+    int jets[2] = {0, 0}, sources = 0;  // stars with a jet (NB_JET_JET, NB_JET_PROTO); the stars depth[1] is for
     int ray_group = 1, fuv_group = 16;  // measured best at 192^3-256^3 (nb_set_tuning)
     int tile_order = 0;
     int front_cull = 1;                 // apply_front skips the stars that cannot change a segment
@@ -166,8 +167,17 @@ long long hydro_columns(const nb_desc& d) {
 }
 
 // planes per hydro tile of the single-instance stages (no_sources: a stirring-phase stage)
-int chosen_depth(const nb_instance* h, bool no_sources) { return h->depth[!no_sources && h->hc.wind_f > 0.0f]; }
+int chosen_depth(const nb_instance* h, bool no_sources) { return h->depth[!no_sources && h->sources > 0]; }
 int chunk_depth(const nb_instance* h, bool no_sources) { return h->chunk_set ? h->chunk_i : chosen_depth(h, no_sources); }
+
+// the stars that work on single cells of a stage, with winds or jets, and the depth for them
+void choose_depth(nb_instance* h) {
+    const NbConst& c = h->hc;
+    const int n = c.wind_f > 0.0f ? h->nstars : (c.jet > 0.0 ? h->jets[0] : 0) + (c.jet_proto > 0.0 ? h->jets[1] : 0);
+    if (n == h->sources) return;
+    h->sources = n;
+    h->depth[1] = nb_hydro_depth(h->d.nx, hydro_columns(h->d), sm_count(), n);
+}
 
 float* plane(nb_instance* h, int p) { return h->d.f.stage + (long long)p * h->ncell; }
 
@@ -494,6 +504,7 @@ NB_EXPORT int nb_set_live(nb_handle h, const nb_live* L) {
     c.plane_lum_f = (float)L->plane_fuv;
     c.pre_amp = L->pre_amp;
     c.drive_main = L->drive_main;
+    choose_depth(h);
     return upload_const(h);
 }
 
@@ -524,9 +535,14 @@ NB_EXPORT int nb_set_stars(nb_handle h, const nb_star* s, int n) {
         tmp[i].kind = s[i].kind; tmp[i].jkind = s[i].jkind;
     }
     if (n > 0) CK(h, cudaMemcpyAsync(h->stars, tmp, sizeof(NbStarDev) * n, cudaMemcpyHostToDevice, h->stream));
-    if (n != h->nstars) h->depth[1] = nb_hydro_depth(h->d.nx, hydro_columns(h->d), sm_count(), n);
     h->nstars = n;
     h->hc.nstars = n;
+    h->jets[0] = h->jets[1] = 0;
+    for (int i = 0; i < n; ++i) {
+        h->jets[0] += s[i].jkind == NB_JET_JET;
+        h->jets[1] += s[i].jkind == NB_JET_PROTO;
+    }
+    choose_depth(h);
     return upload_const(h);
 }
 
@@ -1212,7 +1228,7 @@ NB_EXPORT int nb_batch_create(const nb_handle* hs, const int* ion_every, int n, 
     for (auto* h : b->inst) planes += (double)hydro_columns(h->d) * h->d.nx;
     for (int i = 0; i < n; ++i) {
         nb_instance* h = b->inst[i];
-        const int depth = nb_hydro_depth_batch(planes, b->grid, h->hc.wind_f > 0.0f ? h->nstars : 0);
+        const int depth = nb_hydro_depth_batch(planes, b->grid, h->sources);
         bi[i] = NbBatchInst{h->c, h->st, h->stars, h->sw, h->nstars, 1, h->front_bounds};
         L1[i] = stage_desc(h, false, depth);
         L2[i] = stage_desc(h, true, depth);

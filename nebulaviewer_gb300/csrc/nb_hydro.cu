@@ -295,16 +295,17 @@ int nb_hydro_tile_j() { return HYDRO_TJ; }
 // The i-chunk depth of a stage alone on the GPU: blocks = columns x chunks run in rounds of `sms` x
 // HYDRO_MINB, each of the depth's planes and four halo planes (and about half a plane to start); a
 // last round with fewer blocks on an SM has cheaper planes.  The blocks are as long as one another but
-// for the winds: `winds` stars (none without winds) add HYDRO_WIND of a plane each where a warp has an
-// ionized cell, and the ionized gas may fill one block and miss the next, so a block's share of it is
-// time at the end that no other block fills.  The least time over all chunk counts.
+// for the winds and jets: `sources` stars with one add HYDRO_WIND of a plane each where a warp has an
+// ionized cell or one in a jet's reach, and that gas may fill one block and miss the next, so a block's
+// share of it is time at the end that no other block fills.  The least time over all chunk counts.
 // With a fixed depth of 20 a small grid left SMs idle for 24 serial planes and the last round was
 // often nearly empty: stages 1 + 2 (fast) at 64^3 76 -> 33 us, 128^3 96 -> 88, 192^3 251 -> 235,
 // 256^3 523 -> 502 (depths 4, 15, 48, 37).  Without the winds in it the rule gave one chunk a column at
 // 384^3 for any stars, and the GPU then waited for the few columns in the ionized gas: stages 1 + 2 there
 // with 6 / 24 / 64 / 256 stars 1657 / 2100 / 3429 / 11557 -> 1625 / 1662 / 1814 / 3287 us (depths 96, 35,
 // 24, 12), at 256^3 with 256 stars 2046 -> 1301 (37 -> 8); exact build, 256^3, 24 stars 1219 -> 1167.
-int nb_hydro_depth(int nx, long long columns, int sms, int winds) {
+// Eight stars with jets and no winds, 200^3: 419 -> 336 us (67 -> 20).
+int nb_hydro_depth(int nx, long long columns, int sms, int sources) {
     int best = nx;
     double least = 0.0;
     for (int n = 1, last = 0; n <= nx; ++n) {
@@ -314,7 +315,7 @@ int nb_hydro_depth(int nx, long long columns, int sms, int winds) {
         const long long blocks = columns * ((nx + depth - 1) / depth), round = (long long)sms * HYDRO_MINB;
         const long long rest = blocks % round;
         const double t = ((double)(blocks / round) + HYDRO_PLANE[(rest + sms - 1) / sms]) * (depth + 4.5) +
-                         HYDRO_WIND * winds * depth;
+                         HYDRO_WIND * sources * depth;
         if (least == 0.0 || t < least) {
             least = t;
             best = depth;
@@ -327,10 +328,10 @@ int nb_hydro_depth(int nx, long long columns, int sms, int winds) {
 // The depth of a batch's stages, whose persistent blocks (`slots` of them) take tiles in turn: deep
 // chunks convert fewer halo planes (4.5 per chunk), shallow ones end together (half a chunk idle at the
 // end, and a chunk's wind work, as above); the sum is least at the depth whose square is 9 planes' worth
-// of each block's share, less by the instance's own winds (a batch step of seven 128^3 with one star and a
+// of each block's share, less by the instance's own sources (a batch step of seven 128^3 with one star and a
 // 96^3 with 256 stars 2438 -> 1243 us; 1413 with the most windy instance's depth for all).
-int nb_hydro_depth_batch(double column_planes, int slots, int winds) {
-    const double d = std::sqrt(9.0 * column_planes / (slots > 0 ? slots : 1) / (1.0 + 2.0 * HYDRO_WIND * winds));
+int nb_hydro_depth_batch(double column_planes, int slots, int sources) {
+    const double d = std::sqrt(9.0 * column_planes / (slots > 0 ? slots : 1) / (1.0 + 2.0 * HYDRO_WIND * sources));
     return d < 2.0 ? 2 : (d > 128.0 ? 128 : (int)d);
 }
 

@@ -232,9 +232,10 @@ __device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap* map, int c0, 
 // ------------------------------------------------------------------ launchers (nb_*.cu)
 cudaError_t nb_launch_hydro(const HydroLaunch& L, int solver, int limiter, cudaStream_t s);
 int nb_hydro_tile_j();
-// i-chunk depth of a stage alone on `sms` SMs, and of the batched stage on `slots` blocks; winds: stars with winds
-int nb_hydro_depth(int nx, long long columns, int sms, int winds);
-int nb_hydro_depth_batch(double column_planes, int slots, int winds);
+// i-chunk depth of a stage alone on `sms` SMs, and of the batched stage on `slots` blocks; sources: stars with
+// winds or jets
+int nb_hydro_depth(int nx, long long columns, int sms, int sources);
+int nb_hydro_depth_batch(double column_planes, int slots, int sources);
 int nb_hydro_idx32(long long ncell);     // the stage's 32-bit offsets reach every cell of a grid this large
 // Batches of up to NB_BATCH_PARAM_MAX instances (32-bit cell offsets) hand the persistent stage
 // kernel their stage records as one kernel parameter (28 KB of the 32 KB parameter space): the

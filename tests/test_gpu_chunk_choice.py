@@ -63,3 +63,28 @@ def test_the_chosen_depth_is_not_pinned(sim, monkeypatch):
     monkeypatch.setattr(at, "_measure", lambda s, knob, steps: 1.0 + abs(at.get(s, knob) - 24))
     at.autotune(sim, knobs=["chunk_i"], use_cache=False)
     assert depths(sim) == [24, 24]
+
+
+def test_the_chosen_depth_counts_jets(sim):
+    """stars with jets alone make some tiles slower too; jets of no strength and stars without one do not"""
+    from nebulaviewer_gb300 import autotune as at
+    chosen = depths(sim)
+    sim.P["wind"] = 0.0
+    sim.step(1)
+    assert at.get(sim, "chunk_i") == chosen[1]
+    sim.P["jet"] = 300.0
+    sim.step(1)
+    assert at.get(sim, "chunk_i") == chosen[1]        # no star has a jet
+    sim.jkinds = ["jet"] * 64
+    sim.step(1)
+    assert at.get(sim, "chunk_i") == chosen[0]
+    sim.P["jet"] = 0.0
+    sim.step(1)
+    assert at.get(sim, "chunk_i") == chosen[1]
+    sim.jkinds = ["proto"] * 64
+    sim.P["jet_proto"] = 300.0
+    sim.step(1)
+    assert at.get(sim, "chunk_i") == chosen[0]
+    sim.jkinds = ["none"] * 64
+    sim.step(1)
+    assert at.get(sim, "chunk_i") == chosen[1]
