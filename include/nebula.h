@@ -327,7 +327,7 @@ int nb_profile_read(nb_handle h, double ms[NB_PROF_KINDS], long long count[NB_PR
  * instances where none was set; order 0).  While none is set nb_get_tuning gives the chosen i-chunk, and
  * setting that value leaves the choice to the library.  The hydro
  * result does not depend on them; the ray sums only through their rounding.  NB_TUNE_FRONT_CULL
- * (default 1; up to 32 stars): the front pass first bounds each star's front radius and then
+ * (default 1; up to 32 stars): the ray cast bounds each star's front radius, and the front pass
  * leaves out, per 32-cell segment of a row, the stars that cannot change its ionized fraction or
  * front distance; NB_TUNE_FUV_CUT (default 1): a FUV ray stops once its optical depth passes 120,
  * where exp(-tau) is 0.0f for good, and writes 0 to its remaining bins.  The result is the same

@@ -20,9 +20,12 @@
 // table lies in bricks of 4 u x 4 r, one line each (a ray still writes whole 32-byte sectors), the
 // rays of a brick are cast together, and a warp of the apply takes 4 x 2 x 4 cells instead of 32
 // along k: 21 lines per cell group and star instead of 48.  apply_fuv at 64^3 / 192^3 / 256^3 /
-// 384^3 with six stars: 30 / 256 / 563 / 1954 -> 18 / 177 / 395 / 1298 us (cells alone 458 at
-// 256^3), now issue bound (88%); cast_fuv with its pack 630 -> 590 us at 256^3 (whole pairs where
-// a ray fills its last bins), level below 128^3.
+// 384^3 with six stars: 29 / 262 / 563 / 1954 -> 24 / 178 / 396 / 1299 us (cells alone 458 at
+// 256^3), now issue bound (88%); cast_fuv with its pack 630 -> 589 us at 256^3 (whole pairs where
+// a ray fills its last bins), level at 128^3 and dearer below, where the table keeps the plain order
+// (nb_fuv_bricks).  The cast is bound by L1 (90% of its data pipe) and by the chain of a segment (loads,
+// scan, ballots).  The pack keeps to 8 B a cell, stage planes 0-1, because a render pack's voxels lie in
+// planes 2-3: each cell packed with its upper neighbour (four 16-byte gathers a sample) was 3% faster.
 #include "nb_rayutil.cuh"
 
 namespace {

@@ -240,7 +240,7 @@ cudaError_t run_kernel(const HydroLaunch& L, cudaStream_t s) {
     auto kern = hydro_stage_kernel<SOLVER, LIM, TJ, STAGE2, I32>;
     const int smem = HydroSmem<TJ>::bytes(L.nstars_host);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess)                        // the largest shared-memory carveout: 2 blocks of 108 KB (4 of 57) per SM
+    if (e == cudaSuccess)                        // the largest shared-memory carveout: 2 blocks of 112 KB (fast), 4 of 57 (exact) per SM
         e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return e;
     const int blocks = L.tiles_k * L.tiles_j * L.n_chunks;

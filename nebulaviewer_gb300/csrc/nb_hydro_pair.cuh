@@ -19,10 +19,12 @@
 // of two warps, done a step ahead.  128 registers, 112 KB of shared memory, two blocks per SM at any
 // number of stars.
 //
-// Bound: instruction issue at 16 warps a SM (issue active ~60%; barrier, shared-memory and fixed
-// latencies about equal), not bytes and not one pipe: 320 / 340 thread instructions a cell where pairs
-// of components took 528 / 559.  Measured at 256^3 (sheet, 20-plane chunks; 242 and 261 with the chosen depth): stage 1 309 -> 252 us,
-// stage 2 338 -> 271 us (2.40 and 3.22 TB/s of their 36 and 52 B a cell); 192^3 145 -> 121, 160 -> 130 us.
+// Bound: the shared-memory data pipe, 81 / 79% of its peak wavefronts in stage 1 / 2 (a 16-byte access is four
+// a warp), with 16 warps a SM to hide it: issue is 56% and DRAM 31 / 42%; a warp waits on fixed latencies
+// 1.2 cycles an instruction, on shared memory 0.9, on the barrier 0.9.  313 / 337 thread instructions a cell where
+// pairs of components took 528 / 559.  Measured at 256^3 (sheet, chosen depth of 37 planes): stage 1 309 -> 243 us,
+// stage 2 338 -> 260 us (2.49 and 3.36 TB/s of their 36 and 52 B a cell); 192^3 145 -> 115, 160 -> 123 us.
+// Grids of up to 8 rows leave half a tile idle: 512 x 8 x 512 110 -> 131 us for both stages.
 // Tried on this tile and slower or level: the own cells' values read again from global memory (one
 // address instruction and a pointer load per access, +12%), shuffles along k (+3%), the march unrolled
 // by two (instructions -5%, instruction fetch stalls +), a ninth and tenth warp for the edge work (96

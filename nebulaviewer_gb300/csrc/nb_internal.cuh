@@ -240,7 +240,8 @@ int nb_hydro_idx32(long long ncell);     // the stage's 32-bit offsets reach eve
 // Batches of up to NB_BATCH_PARAM_MAX instances (32-bit cell offsets) hand the persistent stage
 // kernel their stage records as one kernel parameter (28 KB of the 32 KB parameter space): the
 // kernel then reads a record's fields from the constant bank, as the single-instance kernel reads
-// its own, and fits 64 registers (4 blocks / SM) where records read from global memory need 80.
+// its own, and fits its registers: the exact build's 64 (4 blocks / SM) where records read from global
+// memory need 80, the fast build's 128 (2 blocks / SM) where those spill up to 56 bytes.
 #define NB_BATCH_PARAM_MAX 128
 struct NbBatchRecords {
     HydroLaunch L[NB_BATCH_PARAM_MAX];

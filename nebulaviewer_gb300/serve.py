@@ -159,9 +159,9 @@ class _Slot:
 
 
 # Instances of at least this many cells are stepped alone (Sim.step) rather than in the batch:
-# 8 Mi cells is ~2.7 waves of the stage kernels' resident 32 x 8 x 20-cell tiles on 152 SMs, past
-# which a batch no longer fills idle SMs and its kernels cost ~5% more per cell than the
-# single-instance ones (measured on the served mix: 96^3-320^3 snapshots).
+# past 8 Mi cells an instance's tiles fill the 152 SMs for several rounds, a batch fills no idle SMs and
+# its kernels cost ~5% more per cell than the single-instance ones (measured on the served mix:
+# 96^3-320^3 snapshots).
 SOLO_CELLS = 8 * 2 ** 20
 
 
